@@ -113,6 +113,8 @@ struct cmpmc_gpu_ctx {
     int stage_tables = 1;                               // pool forms: decay CDF tables staged in shared memory
     uint32_t pool_ring_cap = 1024;                      // pending phonons per warp (warp pool)
     uint32_t sm_ring_cap = 1u << 17;                    // pending phonons per block (SM-phase pool)
+    bool pool_dense = false;                            // a spread small batch overflowed its rings: one block
+                                                        // per 512 units and full rings from then on
     uint32_t sm_film_cap = 8192;                        // film records per block and phase (SM-phase pool)
     DevBuf pool_ring, pool_film;                        // warp pool: per-warp rings and film buffers
     uint64_t queue_cap = 1ull << 24;                    // Luke-phonon queue entries (64 B each)
@@ -173,7 +175,8 @@ std::vector<uint64_t> graph_key_of(const cmpmc_gpu_ctx* ctx, const cmpmc_run_des
                                static_cast<uint64_t>(d->form), static_cast<uint64_t>(ctx->tpb),
                                static_cast<uint64_t>(ctx->bps), ctx->stack_cap_batched, ctx->hit_cap,
                                static_cast<uint64_t>(ctx->pool), static_cast<uint64_t>(ctx->stage_tables),
-                               ctx->sm_ring_cap, ctx->sm_film_cap, ctx->pool_ring_cap};
+                               ctx->sm_ring_cap, ctx->sm_film_cap, ctx->pool_ring_cap,
+                               static_cast<uint64_t>(ctx->pool_dense)};
     for (const DevBuf* b : {&ctx->stack, &ctx->cstack, &ctx->hit_stage, &ctx->hit_key, &ctx->counters, &ctx->ev_stats,
                             &ctx->ev_nhits, &ctx->offsets, &ctx->hits_out, &ctx->total, &ctx->unit_event,
                             &ctx->ev_offsets, &ctx->ev_stats2, &ctx->partials, &ctx->cursor, &ctx->pool_ring,
@@ -224,11 +227,13 @@ bool sm_pool(const cmpmc_gpu_ctx* ctx) { return ctx->pool == 1 || ctx->pool == 3
 int pool_fp64(const cmpmc_gpu_ctx* ctx) { return ctx->pool == 3 ? 1 : 0; }
 
 // grid of a pool launch over `units` units: one block per SM (SM-phase pool; 512 threads in
-// FP32, 768 in FP64), or the occupancy's 128-thread blocks (warp pool), never more than the
-// units can start
+// FP32, 768 in FP64) from the first units on, since a unit's lineage runs on its block alone
+// (a block per 512 units left 108 of 148 SMs without work at 20,300 units: 45 against 26 ms;
+// 100 units 10.8 against 8.5 ms); or the occupancy's 128-thread blocks (warp pool), never
+// more than the units can start
 int pool_grid(cmpmc_gpu_ctx* ctx, uint64_t units, uint64_t* grid) {
     if (sm_pool(ctx)) {
-        const uint64_t per = static_cast<uint64_t>(sm_pool_threads(pool_fp64(ctx)));
+        const uint64_t per = ctx->pool_dense ? static_cast<uint64_t>(sm_pool_threads(pool_fp64(ctx))) : 1;
         *grid = std::max<uint64_t>(1, std::min<uint64_t>(ctx->num_sms, (units + per - 1) / per));
         return CMPMC_OK;
     }
@@ -241,10 +246,23 @@ int pool_grid(cmpmc_gpu_ctx* ctx, uint64_t units, uint64_t* grid) {
     return CMPMC_OK;
 }
 
-// ring and film buffers for launches of up to `grid` blocks
-int ensure_pool_buffers(cmpmc_gpu_ctx* ctx, uint64_t grid) {
+// ring entries per block of an SM-phase pool launch: the configured capacity is for a block
+// with one unit per thread; blocks that start with fewer units get the same room per unit (a
+// power of two, at least 4,096), so a small batch does not hold a gigabyte of rings
+uint32_t sm_ring_entries(const cmpmc_gpu_ctx* ctx, uint64_t units, uint64_t grid) {
+    if (ctx->pool_dense) return ctx->sm_ring_cap;
+    const uint64_t threads = static_cast<uint64_t>(sm_pool_threads(pool_fp64(ctx)));
+    const uint64_t per_block = (std::max<uint64_t>(units, 1) + grid - 1) / grid;
+    uint32_t cap = std::min<uint32_t>(ctx->sm_ring_cap, 4096);
+    while (cap < ctx->sm_ring_cap && cap / 2 * threads < ctx->sm_ring_cap * per_block) cap *= 2;
+    return cap;
+}
+
+// ring and film buffers for launches of up to `grid` blocks and `units` units
+int ensure_pool_buffers(cmpmc_gpu_ctx* ctx, uint64_t grid, uint64_t units) {
     if (sm_pool(ctx)) {
-        CK(ctx->pool_ring.ensure(grid * ctx->sm_ring_cap * sm_pool_entry_bytes(pool_fp64(ctx))), "alloc block rings");
+        CK(ctx->pool_ring.ensure(grid * sm_ring_entries(ctx, units, grid) * sm_pool_entry_bytes(pool_fp64(ctx))),
+           "alloc block rings");
         CK(ctx->pool_film.ensure(grid * ctx->sm_film_cap * sm_pool_film_bytes(pool_fp64(ctx))), "alloc film buffers");
     } else {
         CK(ctx->pool_ring.ensure(grid * 4 * ctx->pool_ring_cap * pool_ring_entry_bytes()), "alloc warp rings");
@@ -256,7 +274,8 @@ int ensure_pool_buffers(cmpmc_gpu_ctx* ctx, uint64_t grid) {
 cudaError_t launch_pool(cmpmc_gpu_ctx* ctx, const RunArgs& a, uint64_t grid, const QPhonon* queue, cudaStream_t s) {
     const uint32_t* ue = ctx->unit_event.as<uint32_t>();
     if (sm_pool(ctx))
-        return launch_sm_pool_fp32(ctx->L, ctx->cdf_f, ctx->D, a, ctx->pool_ring.p, ctx->sm_ring_cap, ctx->pool_film.p,
+        return launch_sm_pool_fp32(ctx->L, ctx->cdf_f, ctx->D, a, ctx->pool_ring.p,
+                                   sm_ring_entries(ctx, a.n_events, grid), ctx->pool_film.p,
                                    ctx->sm_film_cap, ue, queue, ctx->stage_tables, pool_fp64(ctx),
                                    static_cast<int>(grid), s);
     return launch_pool_fp32(ctx->L, ctx->cdf_f, ctx->D, a, ctx->pool_ring.p, ctx->pool_ring_cap, ctx->pool_film.p, ue,
@@ -266,10 +285,38 @@ cudaError_t launch_pool(cmpmc_gpu_ctx* ctx, const RunArgs& a, uint64_t grid, con
 // after an overflow of a pool's ring or film buffer: more room for the rerun
 void grow_pool(cmpmc_gpu_ctx* ctx, unsigned err) {
     if (err & kErrQueue) {
-        if (sm_pool(ctx)) ctx->sm_ring_cap = std::min<uint32_t>(ctx->sm_ring_cap * 4, 1u << 24);
+        if (sm_pool(ctx) && !ctx->pool_dense) ctx->pool_dense = true;
+        else if (sm_pool(ctx)) ctx->sm_ring_cap = std::min<uint32_t>(ctx->sm_ring_cap * 4, 1u << 24);
         else ctx->pool_ring_cap = std::min<uint32_t>(ctx->pool_ring_cap * 4, 1u << 20);
     }
     if ((err & kErrFilmQueue) && sm_pool(ctx)) ctx->sm_film_cap = std::min<uint32_t>(ctx->sm_film_cap * 2, 1u << 20);
+}
+
+// Launch shape of a thread-per-unit kernel (plain, inline, adjoint and charge kernels). A unit
+// is one serial chain of thousands of steps, and the lanes of a warp that hold units wait for
+// each other's branches, so a batch that cannot fill the chip runs fewer units per warp: as
+// many lanes as it takes to give every resident warp work, never more warps than are resident.
+// `late` (percent) lets that share of the units beyond the resident warps start late on a
+// freed lane instead of adding a lane to every warp: it pays where the lengths of the units
+// differ by several times their mean (plain form: 2,000 events on 1,776 warps take 77 ms on
+// one lane and 88 ms on two), not where they are alike (carriers: 115 ms against 99 ms).
+// Measured against 32 lanes of fewer warps: 2,000 plain phonon events 154 -> 77 ms, 203 plain
+// mixed events 507 -> 230 ms, 4,000 carriers 124 -> 99 ms, adjoint of 20,000 primaries
+// 132 -> 111 ms, 50,000 inline primaries 100 -> 97 ms.
+struct Spread {
+    uint64_t grid;   // blocks
+    uint32_t lanes;  // lanes of each warp that take units
+};
+constexpr uint64_t kLatePlain = 25, kLateNone = 0;
+Spread spread_units(uint64_t units, uint64_t max_blocks, int tpb, uint64_t late) {
+    const uint64_t wpb = static_cast<uint64_t>(tpb) / 32;
+    const uint64_t warps = std::max<uint64_t>(1, max_blocks * wpb);
+    const uint64_t room = warps * (100 + late) / 100;
+    units = std::max<uint64_t>(units, 1);
+    Spread r;
+    r.lanes = static_cast<uint32_t>(std::min<uint64_t>(32, (units + room - 1) / room));
+    r.grid = std::max<uint64_t>(1, std::min<uint64_t>(max_blocks, (units + r.lanes * wpb - 1) / (r.lanes * wpb)));
+    return r;
 }
 
 // Device counters of the batched charge form (reset per phase except next_carrier)
@@ -300,8 +347,8 @@ int run_charges_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a,
         bps_ch = std::max(bps_ch, 1);
     }
     const uint64_t grid_ph = static_cast<uint64_t>(ctx->num_sms) * bps_ph;
-    const uint64_t grid_ch = std::max<uint64_t>(
-        1, std::min<uint64_t>(static_cast<uint64_t>(ctx->num_sms) * bps_ch, (n_ch + tpb - 1) / tpb));
+    const Spread sp_ch = spread_units(n_ch, static_cast<uint64_t>(ctx->num_sms) * bps_ch, tpb, kLateNone);
+    const uint64_t grid_ch = sp_ch.grid;
     const uint64_t resume_cap = grid_ch * tpb * 9;  // a carrier and up to 8 knock-ons per thread
     uint64_t q_cap = std::max<uint64_t>(ctx->queue_cap, 64);
     // collections with a release mode (BulkDebye / ElectrodeFilm) wait in a record buffer
@@ -442,7 +489,7 @@ int run_charges_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a,
             }
         };
         if (pool) {
-            const int st = ensure_pool_buffers(ctx, grid_pool);
+            const int st = ensure_pool_buffers(ctx, grid_pool, ~0ull >> 32);  // the rounds' sizes vary
             if (st != CMPMC_OK) return st;
         }
         // one pool launch over `units` units: the primaries (queue == nullptr) or a queue
@@ -495,8 +542,10 @@ int run_charges_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a,
             ca.resume_in = r_in;
             ca.n_resume_in = n_resume;
             ca.resume_out = r_out;
+            a.lanes = sp_ch.lanes;
             CK(launch_charges_fp32(ctx->L, ctx->cdf_f, ctx->D, a, ca, static_cast<int>(grid_ch), tpb, s),
                "charge launch");
+            a.lanes = 32;
             ++launches;
             CK(cudaMemcpyAsync(hbuf + sizeof(Counters), cc, sizeof(ChargeCounters), cudaMemcpyDeviceToHost, s),
                "copy counters");
@@ -562,7 +611,7 @@ int run_charges_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a,
         split_over = split_over || (!pool && (hc.err & (kErrQueue | kErrFilmQueue)) != 0);
         if (!stack_over && !hits_over && !queue_over && !split_over && !ring_over) break;
         if (ring_over) grow_pool(ctx, hc.err);
-        if (attempt >= 8) return fail(ctx, CMPMC_ERR_CAPACITY, "device stack, hit or queue overflow persists");
+        if (attempt >= 9) return fail(ctx, CMPMC_ERR_CAPACITY, "device stack, hit or queue overflow persists");
         if (stack_over) stack_cap = std::min<uint32_t>(stack_cap * 8, 1u << 20);
         if (hits_over) hit_cap = hc.hit_count + hc.hit_count / 16 + 1024;
         if (queue_over) {
@@ -788,10 +837,6 @@ int run_pool_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a, ui
         hc = Counters{};
     }
     uint64_t grid = 1;
-    {
-        const int st = pool_grid(ctx, n_ph, &grid);
-        if (st != CMPMC_OK) return st;
-    }
     CK(ctx->ev_stats2.ensure(std::max<uint64_t>(n, 1) * sizeof(cmpmc_sim_stats)), "alloc event stats");
     CK(ctx->ev_nhits.ensure(std::max<uint64_t>(n, 1) * 8), "alloc event hit counts");
     CK(ctx->ev_offsets.ensure((n + 1) * 8), "alloc event offsets");
@@ -820,7 +865,8 @@ int run_pool_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a, ui
     for (int attempt = 0;; ++attempt) {
         if (!d->keep_hits) hit_cap = 1;
         {
-            const int st = ensure_pool_buffers(ctx, grid);
+            int st = pool_grid(ctx, n_ph, &grid);
+            if (st == CMPMC_OK) st = ensure_pool_buffers(ctx, grid, n_ph);
             if (st != CMPMC_OK) return st;
         }
         CK(ctx->hit_stage.ensure(hit_cap * sizeof(cmpmc_sensor_hit)), "alloc hit staging");
@@ -845,7 +891,7 @@ int run_pool_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a, ui
         const bool ring_over = (hc.err & (kErrQueue | kErrFilmQueue)) != 0;
         const bool hits_over = d->keep_hits && hc.hit_count > hit_cap;
         if (!ring_over && !hits_over) break;
-        if (attempt >= 6) return fail(ctx, CMPMC_ERR_CAPACITY, "pool ring or hit buffer overflow persists");
+        if (attempt >= 7) return fail(ctx, CMPMC_ERR_CAPACITY, "pool ring or hit buffer overflow persists");
         if (ring_over) grow_pool(ctx, hc.err);
         if (hits_over) hit_cap = hc.hit_count + hc.hit_count / 16 + 1024;
         hc.err = 0;
@@ -1199,6 +1245,7 @@ int cmpmc_gpu_configure_pool(cmpmc_gpu_ctx* ctx, int form, uint32_t ring_capacit
         return fail(ctx, CMPMC_ERR_INVALID, "ring capacity: a power of two, at least 64");
     drop_graph(ctx);
     ctx->pool = form;
+    ctx->pool_dense = false;
     if (ring_capacity) {
         if (form == 1 || form == 3) ctx->sm_ring_cap = std::max<uint32_t>(ring_capacity, 2048);  // a block appends up to 2 x 512 at once
         else ctx->pool_ring_cap = ring_capacity;
@@ -1362,6 +1409,7 @@ int cmpmc_gpu_run_events(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, cmpmc_run_
     a.first_event = d->first_event;
     a.keep_hits = d->keep_hits;
     a.seed = d->seed;
+    a.lanes = 32;
     if (d->kaplan_surrogate && batched) {
         const int st = ensure_surrogate(ctx);
         if (st != CMPMC_OK) return st;
@@ -1469,10 +1517,11 @@ int cmpmc_gpu_run_events(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, cmpmc_run_
             CK(batched ? batched_fp32_occupancy(ctx->tpb, &bps) : plain_fp64_occupancy(ctx->tpb, &bps), "occupancy");
             bps = std::max(bps, 1);
         }
-        uint64_t grid = static_cast<uint64_t>(ctx->num_sms) * bps;
-        grid = std::min<uint64_t>(grid, (std::max<uint64_t>(units, 1) + ctx->tpb - 1) / ctx->tpb);
-        grid = std::max<uint64_t>(grid, 1);
-        const uint64_t slots = grid * ctx->tpb;
+        const Spread sp = spread_units(units, static_cast<uint64_t>(ctx->num_sms) * bps, ctx->tpb,
+                                       batched ? kLateNone : kLatePlain);
+        const uint64_t grid = sp.grid;
+        a.lanes = sp.lanes;
+        const uint64_t slots = grid * (ctx->tpb / 32) * sp.lanes;
         const size_t stack_entry = batched ? batched_stack_entry_bytes() : sizeof(GTrack);
 
         CK(ctx->ev_stats.ensure(std::max<uint64_t>(units, 1) * sizeof(cmpmc_sim_stats)), "alloc unit stats");
@@ -1724,10 +1773,10 @@ int cmpmc_gpu_adjoint(cmpmc_gpu_ctx* ctx, const cmpmc_adjoint_desc* d, cmpmc_adj
         CK(adjoint_fp32_occupancy(ctx->tpb, &bps), "occupancy");
         bps = std::max(bps, 1);
     }
-    uint64_t grid = static_cast<uint64_t>(ctx->num_sms) * bps;
-    grid = std::min<uint64_t>(grid, (std::max<uint64_t>(units, 1) + ctx->tpb - 1) / ctx->tpb);
-    grid = std::max<uint64_t>(grid, 1);
-    const uint64_t slots = grid * ctx->tpb;
+    const Spread sp = spread_units(units, static_cast<uint64_t>(ctx->num_sms) * bps, ctx->tpb, kLateNone);
+    const uint64_t grid = sp.grid;
+    a.lanes = sp.lanes;
+    const uint64_t slots = grid * (ctx->tpb / 32) * sp.lanes;
 
     CK(ctx->ev_stats.ensure(std::max<uint64_t>(units, 1) * sizeof(cmpmc_sim_stats)), "alloc unit stats");
     CK(ctx->ev_nhits.ensure(std::max<uint64_t>(units, 1) * 8), "alloc unit hit counts");

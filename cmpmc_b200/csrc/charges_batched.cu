@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(128, 5) k_charges_fp32(const __grid_constant__
     for (int i = threadIdx.x; i < static_cast<int>(sizeof(FCLat) / 4); i += blockDim.x)
         reinterpret_cast<uint32_t*>(&sL)[i] = reinterpret_cast<const uint32_t*>(&Lp)[i];
     __syncthreads();
+    if (!lane_active(a.lanes)) return;
     const FCLat& L = sL;
     Carrier k;
     CStats st{};

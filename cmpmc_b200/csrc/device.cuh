@@ -79,7 +79,17 @@ struct RunArgs {
     // wavefront split: a track that has taken this many steps in the current phase is parked
     // in `reemit` (next phase) on a substream derived from its own (0: no limit)
     uint32_t phase_steps;
+    // thread-per-unit kernels: lanes of each warp that take units (see spread_lanes)
+    uint32_t lanes;
 };
+
+// The thread-per-unit kernels run units on the first `lanes` lanes of every warp; the active
+// threads are numbered without gaps, so the per-thread stacks need `lanes` slots per warp.
+__device__ __forceinline__ bool lane_active(uint32_t lanes) { return (threadIdx.x & 31u) < lanes; }
+__device__ __forceinline__ uint64_t lane_slot(uint32_t lanes) {
+    const uint64_t warp = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
+    return warp * lanes + (threadIdx.x & 31u);
+}
 
 // Phonon queue entry of the batched forms (64 B): Luke phonons of the charge form and
 // film re-emissions of the wavefront split. ev == kQEmpty marks a slot that was reserved

@@ -20,6 +20,7 @@
 // is the Kaplan film cascade (so the ledger closes to rounding). A reflected track is
 // moved 10 nm inward (the reference moves it 1e-11 m, below FP32 resolution at the wall).
 #define CMPMC_DEVICE_FAST_MATH 1
+#include <algorithm>
 #include <type_traits>
 
 #include "device.cuh"
@@ -359,7 +360,7 @@ __device__ __forceinline__ void batched_loop(const FLat& L, const Detector& D, c
                                              const uint32_t* __restrict__ unit_event,
                                              const QPhonon* __restrict__ queue, const AdjArgs& adj,
                                              float* s_w, float* s_hist) {
-    const uint64_t slot = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    const uint64_t slot = lane_slot(a.lanes);
     double refl_buf[kKaplanCap];
     double kwork[4 * kKaplanCap];
     EntryOf<kAdj>* stk = reinterpret_cast<EntryOf<kAdj>*>(a.stack) + slot * a.stack_cap;
@@ -742,6 +743,7 @@ __global__ void __launch_bounds__(128, 6) k_batched_fp32(const __grid_constant__
                                                          const __grid_constant__ Detector D,
                                                          const __grid_constant__ RunArgs a,
                                                          const uint32_t* __restrict__ unit_event) {
+    if (!lane_active(a.lanes)) return;
     const AdjArgs none{};
     batched_loop<false, kSrcInput, kSink, kSur, kSplit, kKin>(L, D, a, unit_event, nullptr, none, nullptr, nullptr);
 }
@@ -752,6 +754,7 @@ __global__ void __launch_bounds__(128, 6) k_queue_fp32(const __grid_constant__ F
                                                        const __grid_constant__ Detector D,
                                                        const __grid_constant__ RunArgs a,
                                                        const QPhonon* __restrict__ queue) {
+    if (!lane_active(a.lanes)) return;
     const AdjArgs none{};
     batched_loop<false, kSrcQueue, true, kSur, kSplit, kKin>(L, D, a, nullptr, queue, none, nullptr, nullptr);
 }
@@ -1604,6 +1607,7 @@ struct SmPoolArgs {
     const uint32_t* unit_event;
     const QPhonon* queue;    // queue units (kQueue kernels)
     int stage_tables;
+    uint32_t share;          // units a warp claims at a time: a small batch is spread over the warps
 };
 
 struct SmShared {
@@ -2170,6 +2174,8 @@ __device__ __noinline__ void sm_film_phase(const typename P::Lat* Lp, const Dete
                                            const typename P::Film* film, uint32_t n_film, SmShared* sh,
                                            typename P::Entry* ring, uint32_t ring_mask, uint32_t r_floor,
                                            unsigned* err) {
+    constexpr uint32_t kWarps = SmShape<P::kThreads>::kWarps;
+    if ((threadIdx.x & 31u) * kWarps >= n_film) return;  // few records: spread over the warps
     double refl_buf[kKaplanCap];
     double kwork[4 * kKaplanCap];
     for (;;) {
@@ -2231,6 +2237,8 @@ __global__ void __launch_bounds__(P::kThreads, 1) k_sm_pool(const __grid_constan
         // ---- transport phase --------------------------------------------------------
         const uint32_t r_floor = vsh->r_head;  // ring slots below it are free
         const uint32_t r_pub = vsh->r_pub;
+        // entries a warp claims at a time: few waiting entries are spread over the warps
+        const uint32_t r_share = (r_pub - r_floor + SmShape<P::kThreads>::kWarps - 1) / SmShape<P::kThreads>::kWarps;
         SmSink<Film, Entry> sink{&sh, film, ring, p.film_cap, ring_mask, r_floor, &err, &a};
         for (;;) {
             uint32_t ft = 0, inp = 0, dry = 0, unpub = 0;
@@ -2254,8 +2262,9 @@ __global__ void __launch_bounds__(P::kThreads, 1) k_sm_pool(const __grid_constan
                 const int rank = __popc(empty & lanemask_lt());
                 uint32_t base = 0, got = 0;
                 if (lane == 0 && vsh->r_head < r_pub) {
-                    base = atomicAdd(&sh.r_head, static_cast<uint32_t>(n_empty));
-                    got = (base < r_pub) ? min(static_cast<uint32_t>(n_empty), r_pub - base) : 0u;
+                    const uint32_t want = min(static_cast<uint32_t>(n_empty), r_share);
+                    base = atomicAdd(&sh.r_head, want);
+                    got = (base < r_pub) ? min(want, r_pub - base) : 0u;
                 }
                 base = __shfl_sync(full, base, 0);
                 got = __shfl_sync(full, got, 0);
@@ -2267,7 +2276,7 @@ __global__ void __launch_bounds__(P::kThreads, 1) k_sm_pool(const __grid_constan
                     st.clear();
                     live = true;
                 }
-                const int need = n_empty - static_cast<int>(got);
+                const int need = min(n_empty - static_cast<int>(got), static_cast<int>(p.share));
                 if (need > 0 && inp) {
                     unsigned long long ub = 0;
                     if (lane == 0) {
@@ -2275,8 +2284,9 @@ __global__ void __launch_bounds__(P::kThreads, 1) k_sm_pool(const __grid_constan
                         if (ub + need >= a.n_events) vsh->input_left = 0;
                     }
                     ub = __shfl_sync(full, ub, 0);
-                    const uint64_t unit = ub + static_cast<uint64_t>(rank - static_cast<int>(got));
-                    if (!live && rank >= static_cast<int>(got) && unit < a.n_events) {
+                    const int at = rank - static_cast<int>(got);
+                    const uint64_t unit = ub + static_cast<uint64_t>(at);
+                    if (!live && at >= 0 && at < need && unit < a.n_events) {
                         if constexpr (kQueue) {
                             const QPhonon q = p.queue[unit];
                             if (q.ev != kQEmpty) {
@@ -2345,7 +2355,7 @@ __global__ void __launch_bounds__(128, 6) k_adjoint_fp32(const __grid_constant__
         s_hist[b] = 0.0f;
     }
     __syncthreads();
-    batched_loop<true>(L, D, a, unit_event, nullptr, adj, s_w, s_hist);
+    if (lane_active(a.lanes)) batched_loop<true>(L, D, a, unit_event, nullptr, adj, s_w, s_hist);
     __syncthreads();
     for (int b = threadIdx.x; b < adj.n_bins; b += blockDim.x)
         if (s_hist[b] != 0.0f) atomicAdd(adj.hist + b, static_cast<double>(s_hist[b]));
@@ -2466,6 +2476,8 @@ cudaError_t launch_sm_pool_fp32(const Lattice& L, const float* cdf_f, const Dete
     p.unit_event = unit_event;
     p.queue = queue;
     p.stage_tables = stage_tables;
+    const uint64_t warps = static_cast<uint64_t>(grid) * (threads / 32);
+    p.share = static_cast<uint32_t>(std::min<uint64_t>(32, std::max<uint64_t>(1, (a.n_events + warps - 1) / warps)));
     if (fp64) {  // the FP64 comparison form: phonon batches, every kinematics mode, full cascades
         if (queue || a.surrogate) return cudaErrorInvalidValue;
         return sm_launch<PF64, false>(L, D, a, p, grid, s);

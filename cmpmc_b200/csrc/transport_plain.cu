@@ -124,7 +124,8 @@ struct PlainCtx {
 };
 
 __global__ void __launch_bounds__(128) k_plain_fp64(const Lattice L, const Detector D, const RunArgs a) {
-    const uint64_t slot = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    if (!lane_active(a.lanes)) return;
+    const uint64_t slot = lane_slot(a.lanes);
     double refl_buf[kKaplanCap];
     double kwork[4 * kKaplanCap];
     PlainCtx ctx;
