@@ -1175,7 +1175,7 @@ int cmpmc_gpu_autotune(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* sample, int rep
     for (int tpb : {64, 128}) {
         int occ = 1;
         CK(charges ? charges_fp32_occupancy(tpb, &occ)
-                   : (batched ? batched_fp32_occupancy(tpb, &occ) : plain_fp64_occupancy(tpb, &occ)),
+                   : (batched ? batched_fp32_occupancy(tpb, &occ) : plain_fp64_occupancy(tpb, sample->charge_offsets != nullptr, &occ)),
            "occupancy");
         occ = std::max(occ, 1);
         int tried[3] = {occ, std::max(1, (3 * occ) / 4), std::max(1, occ / 2)};
@@ -1514,7 +1514,7 @@ int cmpmc_gpu_run_events(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, cmpmc_run_
         a.n_events = units;
         int bps = ctx->bps;
         if (!bps) {
-            CK(batched ? batched_fp32_occupancy(ctx->tpb, &bps) : plain_fp64_occupancy(ctx->tpb, &bps), "occupancy");
+            CK(batched ? batched_fp32_occupancy(ctx->tpb, &bps) : plain_fp64_occupancy(ctx->tpb, has_charges, &bps), "occupancy");
             bps = std::max(bps, 1);
         }
         const Spread sp = spread_units(units, static_cast<uint64_t>(ctx->num_sms) * bps, ctx->tpb,

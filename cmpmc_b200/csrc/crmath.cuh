@@ -42,22 +42,35 @@
 #endif
 #endif
 
-// rare slow paths are kept out of line so the hot kernels stay small
+// The functions are out of line on the device: inlined at every use the FP64 step loops grew
+// to many times the instruction cache, and with few warps per scheduler a quarter of their
+// issue slots waited for instructions.
 #ifdef __CUDACC__
 #define CMPMC_CR_COLD static __host__ __device__ __noinline__
+#define CMPMC_CR_FN static __host__ __device__ __noinline__
 #else
 #define CMPMC_CR_COLD static inline
+#define CMPMC_CR_FN static inline
 #endif
 
 namespace cmpmc_gpu {
 namespace crmath {
 
+// 128 / n rounded, n = 85 .. 171 (the reciprocals of the reduction points of log)
+struct InvC {
+    double v[87];
+    constexpr InvC() : v() {
+        for (int i = 0; i < 87; ++i) v[i] = 128.0 / (85 + i);
+    }
+};
+static constexpr InvC h_invc{};
 static const double h_logc[87][2] = CMPMC_CR_LOGC;
 static const double h_invodd[12][2] = CMPMC_CR_INVODD;
 static const double h_sinc[16][2] = CMPMC_CR_SINC;
 static const double h_cosc[17][2] = CMPMC_CR_COSC;
 #ifdef __CUDACC__
 static __device__ const double d_logc[87][2] = CMPMC_CR_LOGC;
+static __device__ constexpr InvC d_invc{};
 static __constant__ double d_invodd[12][2] = CMPMC_CR_INVODD;
 static __constant__ double d_sinc[16][2] = CMPMC_CR_SINC;
 static __constant__ double d_cosc[17][2] = CMPMC_CR_COSC;
@@ -68,11 +81,13 @@ static __constant__ double d_cosc[17][2] = CMPMC_CR_COSC;
 CMPMC_HD double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 CMPMC_HD double logc_hi(int i) { return __ldg(&d_logc[i][0]); }
 CMPMC_HD double logc_lo(int i) { return __ldg(&d_logc[i][1]); }
+CMPMC_HD double invc(int i) { return __ldg(&d_invc.v[i]); }
 #else
 #define CMPMC_CR_TAB(name) h_##name
 CMPMC_HD double fma_rn(double a, double b, double c) { return ::fma(a, b, c); }
 CMPMC_HD double logc_hi(int i) { return h_logc[i][0]; }
 CMPMC_HD double logc_lo(int i) { return h_logc[i][1]; }
+CMPMC_HD double invc(int i) { return h_invc.v[i]; }
 #endif
 
 struct DD {
@@ -176,8 +191,10 @@ CMPMC_HD bool ziv_ok(double h, double l, double eps) {
 // log(x) correctly rounded for positive finite x; other inputs go to the platform log.
 // Fast path: the same reduction with log1p(r) summed as r - r^2/2 (error-free) plus an
 // FP64 tail, relative error below 2^-64; the double-double path runs only when the
-// rounding test fails (about one call in a thousand).
-CMPMC_HD double log(double x) {
+// rounding test fails (about one call in a thousand). r = t / c = q + ql with q = t (1/c)
+// rounded: the residual t - q c is exact (q has 53 bits, c eight, and q is within two units of
+// t / c), so no division is needed.
+CMPMC_CR_FN double log(double x) {
     if (!(x > 0.0) || !(x < __builtin_huge_val())) return ::log(x);
     uint64_t bits;
     memcpy(&bits, &x, 8);
@@ -196,14 +213,22 @@ CMPMC_HD double log(double x) {
     }
     const int n = static_cast<int>(m * 128.0 + 0.5);
     const double c = n * (1.0 / 128.0);
+    const double rc = invc(n - 85);
     const double t = m - c;
-    const double q = t / c;
-    const double ql = fma_rn(-q, c, t) / c;  // r = q + ql
+    const double q = t * rc;
+    const double ql = fma_rn(-q, c, t) * rc;  // r = q + ql
     const DD z = two_prod(q, q);
     // log1p(q) - q + q^2/2 = q^3 (1/3 - q/4 + q^2/5 - ...), |q| < 2^-7.4, to q^11
-    const double tail = q * z.hi *
-                        (1.0 / 3 + q * (-1.0 / 4 + q * (1.0 / 5 + q * (-1.0 / 6 + q * (1.0 / 7 + q * (-1.0 / 8 +
-                         q * (1.0 / 9 + q * (-1.0 / 10 + q * (1.0 / 11)))))))));
+    double p = 1.0 / 11;
+    p = fma_rn(q, p, -1.0 / 10);
+    p = fma_rn(q, p, 1.0 / 9);
+    p = fma_rn(q, p, -1.0 / 8);
+    p = fma_rn(q, p, 1.0 / 7);
+    p = fma_rn(q, p, -1.0 / 6);
+    p = fma_rn(q, p, 1.0 / 5);
+    p = fma_rn(q, p, -1.0 / 4);
+    p = fma_rn(q, p, 1.0 / 3);
+    const double tail = q * z.hi * p;
     const double ed = static_cast<double>(e);
     const DD A = two_sum(ed * CMPMC_CR_LN2_H42, logc_hi(n - 85));  // ed * head is exact
     const DD B = two_sum(A.hi, q);
@@ -246,16 +271,38 @@ CMPMC_HD double scale2(double v, int k) {
     return (v * f1) * f2;
 }
 
-// exp(x) correctly rounded for |x| < 700 (results in the normal range)
-CMPMC_HD double exp(double x) {
+// exp(x) correctly rounded for |x| < 700 (results in the normal range). Fast path: the same
+// reduction with exp(t), t = r/16, |t| < 0.022, summed as 1 + t + t^2/2 in double-double plus an
+// FP64 tail from t^3/6 (below 2^-19, so its rounding is below 2^-70); the four squarings leave
+// the relative error below 2^-64.
+CMPMC_CR_FN double exp(double x) {
     if (!(fabs(x) < 700.0)) return ::exp(x);
+    const double kd = rint(x * 1.4426950408889634);
+    const DD a = two_sum(x, -kd * CMPMC_CR_LN2_H42);  // kd * head is exact
+    DD t = fast_two_sum(a.hi, a.lo - kd * CMPMC_CR_LN2_T42);
+    t = DD{t.hi * 0.0625, t.lo * 0.0625};
+    const double h = t.hi;
+    double p = 1.0 / 362880;
+    p = fma_rn(h, p, 1.0 / 40320);
+    p = fma_rn(h, p, 1.0 / 5040);
+    p = fma_rn(h, p, 1.0 / 720);
+    p = fma_rn(h, p, 1.0 / 120);
+    p = fma_rn(h, p, 1.0 / 24);
+    p = fma_rn(h, p, 1.0 / 6);
+    const DD z = two_prod(h, h);
+    const DD s = two_sum(1.0, h);
+    const DD u = two_sum(s.hi, 0.5 * z.hi);
+    DD e = fast_two_sum(u.hi, u.lo + s.lo + (t.lo + h * t.lo) + 0.5 * z.lo + h * z.hi * p);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e = dd_mul(e, e);
+    if (ziv_ok(e.hi, e.lo, 0x1p-62)) return scale2(e.hi, static_cast<int>(kd));
     int k;
-    const DD e = exp_dd(DD{x, 0.0}, k);
-    return scale2(e.hi + e.lo, k);
+    const DD v = exp_dd(DD{x, 0.0}, k);
+    return scale2(v.hi + v.lo, k);
 }
 
 // pow(x, y) = exp(y log x) correctly rounded for x > 0 and |y log x| < 700
-CMPMC_HD double pow(double x, double y) {
+CMPMC_CR_FN double pow(double x, double y) {
     if (!(x > 0.0) || !(x < __builtin_huge_val()) || !(fabs(y) < 1e300)) return ::pow(x, y);
     if (y == 0.0 || x == 1.0) return 1.0;
     const DD t = dd_mul_d(log_dd(x), y);
@@ -266,7 +313,7 @@ CMPMC_HD double pow(double x, double y) {
 }
 
 // sqrt(x^2 + y^2) correctly rounded, for |x|, |y| in [2^-400, 2^400] (or one of them 0)
-CMPMC_HD double hypot(double x, double y) {
+CMPMC_CR_FN double hypot(double x, double y) {
     x = fabs(x);
     y = fabs(y);
     if (x < y) {
@@ -285,7 +332,7 @@ CMPMC_HD double hypot(double x, double y) {
 }
 
 // cbrt(x) correctly rounded: one Newton step in double-double from the platform cbrt
-CMPMC_HD double cbrt(double x) {
+CMPMC_CR_FN double cbrt(double x) {
     const double ax = fabs(x);
     if (!(ax > 2.3e-200) || !(ax < 4.3e200)) return ::cbrt(x);
     const double y = ::cbrt(ax);
@@ -333,12 +380,17 @@ CMPMC_HD DD sin_fast(DD r) {
     const DD p3 = two_prod(rh, z.hi);
     const DD r3 = fast_two_sum(p3.hi, p3.lo + rh * z.lo);            // rh^3
     const DD t3 = dd_mul(r3, DD{CMPMC_CR_INV6_HI, CMPMC_CR_INV6_LO});
-    const DD t5 = dd_div(dd_mul(r3, z), DD{120.0, 0.0});
+    const DD t5 = dd_mul(dd_mul(r3, z), dd_tab(CMPMC_CR_TAB(sinc), 2));  // 1/120
     const double zz = z.hi;
-    const double tail7 = rh * zz * zz * zz *
-                         (-1.0 / 5040 + zz * (1.0 / 362880 + zz * (-1.0 / 39916800 + zz * (1.0 / 6227020800.0 +
-                          zz * (-1.0 / 1307674368000.0 + zz * (1.0 / 355687428096000.0 +
-                          zz * (-1.0 / 121645100408832000.0 + zz * (1.0 / 51090942171709440000.0))))))));
+    double p = 1.0 / 51090942171709440000.0;
+    p = fma_rn(zz, p, -1.0 / 121645100408832000.0);
+    p = fma_rn(zz, p, 1.0 / 355687428096000.0);
+    p = fma_rn(zz, p, -1.0 / 1307674368000.0);
+    p = fma_rn(zz, p, 1.0 / 6227020800.0);
+    p = fma_rn(zz, p, -1.0 / 39916800);
+    p = fma_rn(zz, p, 1.0 / 362880);
+    p = fma_rn(zz, p, -1.0 / 5040);
+    const double tail7 = rh * zz * zz * zz * p;
     const double dcos = 1.0 - 0.5 * zz + zz * zz * (1.0 / 24) - zz * zz * zz * (1.0 / 720);
     DD s = two_sum(rh, -t3.hi);
     const DD s2 = two_sum(s.hi, t5.hi);
@@ -352,10 +404,15 @@ CMPMC_HD DD cos_fast(DD r) {
     const DD zsq = two_prod(z.hi, z.hi);
     const DD t4 = dd_mul(DD{zsq.hi, zsq.lo + 2.0 * z.hi * w}, DD{CMPMC_CR_INV24_HI, CMPMC_CR_INV24_LO});
     const double zz = z.hi;
-    const double tail6 = zz * zz * zz *
-                         (-1.0 / 720 + zz * (1.0 / 40320 + zz * (-1.0 / 3628800 + zz * (1.0 / 479001600.0 +
-                          zz * (-1.0 / 87178291200.0 + zz * (1.0 / 20922789888000.0 +
-                          zz * (-1.0 / 6402373705728000.0 + zz * (1.0 / 2432902008176640000.0))))))));
+    double p = 1.0 / 2432902008176640000.0;
+    p = fma_rn(zz, p, -1.0 / 6402373705728000.0);
+    p = fma_rn(zz, p, 1.0 / 20922789888000.0);
+    p = fma_rn(zz, p, -1.0 / 87178291200.0);
+    p = fma_rn(zz, p, 1.0 / 479001600.0);
+    p = fma_rn(zz, p, -1.0 / 3628800);
+    p = fma_rn(zz, p, 1.0 / 40320);
+    p = fma_rn(zz, p, -1.0 / 720);
+    const double tail6 = zz * zz * zz * p;
     const DD c = two_sum(1.0, -0.5 * z.hi);
     const DD c2 = two_sum(c.hi, t4.hi);
     const double lo = c.lo + c2.lo + t4.lo - 0.5 * w + tail6;
@@ -365,7 +422,7 @@ CMPMC_HD DD cos_fast(DD r) {
 CMPMC_CR_COLD double sin_slow(double x);
 CMPMC_CR_COLD double cos_slow(double x);
 
-CMPMC_HD double sin(double x) {
+CMPMC_CR_FN double sin(double x) {
     if (!in_range(x) || x == 0.0) return sin_slow(x);
     int q;
     const DD r = reduce_pio2(x, q);
@@ -374,7 +431,7 @@ CMPMC_HD double sin(double x) {
     return (q & 2) ? -v.hi : v.hi;
 }
 
-CMPMC_HD double cos(double x) {
+CMPMC_CR_FN double cos(double x) {
     if (!in_range(x)) return cos_slow(x);
     int q;
     const DD r = reduce_pio2(x, q);
@@ -426,7 +483,7 @@ CMPMC_CR_COLD void sincos_dd(double x, DD& s, DD& c) {
 
 // acos(x) correctly rounded: one Newton step on cos(y) = x in double-double from the
 // platform acos (|x| = 1 and arguments outside [-1, 1] go to the platform acos).
-CMPMC_HD double acos(double x) {
+CMPMC_CR_FN double acos(double x) {
     if (!(fabs(x) < 1.0)) return ::acos(x);
     const double y0 = ::acos(x);
     DD s, c;
@@ -438,7 +495,7 @@ CMPMC_HD double acos(double x) {
 
 // atan2(y, x) correctly rounded: one Newton step on y cos(t) - x sin(t) = 0 in double-double
 // from the platform atan2 (zeros, infinities and NaNs go to the platform atan2).
-CMPMC_HD double atan2(double y, double x) {
+CMPMC_CR_FN double atan2(double y, double x) {
     if (!(fabs(x) < 1.0 / 0.0) || !(fabs(y) < 1.0 / 0.0) || x == 0.0 || y == 0.0) return ::atan2(y, x);
     const double t0 = ::atan2(y, x);
     DD s, c;
@@ -448,10 +505,28 @@ CMPMC_HD double atan2(double y, double x) {
     return t0 + (f.hi + f.lo) / g;
 }
 
-// both at once
-CMPMC_HD void sincos(double x, double& s, double& c) {
-    s = sin(x);
-    c = cos(x);
+// both at once, from one reduction (the quadrant only exchanges the two kernels' results)
+struct SinCos {
+    double s, c;
+};
+CMPMC_CR_FN SinCos sincos(double x) {
+    if (!in_range(x) || x == 0.0) return SinCos{sin_slow(x), cos_slow(x)};
+    int q;
+    const DD r = reduce_pio2(x, q);
+    const DD a = sin_fast(r), b = cos_fast(r);
+    double s = (q & 1) ? b.hi : a.hi, c = (q & 1) ? a.hi : b.hi;
+    const bool ok_a = ziv_ok(a.hi, a.lo, 0x1p-62), ok_b = ziv_ok(b.hi, b.lo, 0x1p-62);
+    if (!(ok_a && ok_b)) {
+        if (!((q & 1) ? ok_b : ok_a)) {
+            s = sin_slow(x);
+            s = (q & 2) ? -s : s;
+        }
+        if (!((q & 1) ? ok_a : ok_b)) {
+            c = cos_slow(x);
+            c = ((q + 1) & 2) ? -c : c;
+        }
+    }
+    return SinCos{(q & 2) ? -s : s, ((q + 1) & 2) ? -c : c};
 }
 
 }  // namespace crmath

@@ -251,7 +251,7 @@ CMPMC_HD void stats_from_event(const EvStats& e, double injected, cmpmc_sim_stat
 // kernels (launch wrappers return the cudaError_t of the launch)
 cudaError_t launch_plain_fp64(const Lattice& L, const Detector& D, const RunArgs& a, int grid, int block,
                               cudaStream_t s);
-cudaError_t plain_fp64_occupancy(int block, int* blocks_per_sm);
+cudaError_t plain_fp64_occupancy(int block, bool charges, int* blocks_per_sm);
 cudaError_t launch_batched_fp32(const Lattice& L, const float* cdf_f, const Detector& D, const RunArgs& a,
                                 const uint32_t* unit_event, int grid, int block, cudaStream_t s);
 cudaError_t batched_fp32_occupancy(int block, int* blocks_per_sm);

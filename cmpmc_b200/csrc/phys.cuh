@@ -32,6 +32,11 @@ namespace cmpmc_gpu {
 CMPMC_HD double m_log(double x) { return crmath::log(x); }
 CMPMC_HD double m_sin(double x) { return crmath::sin(x); }
 CMPMC_HD double m_cos(double x) { return crmath::cos(x); }
+CMPMC_HD void m_sincos(double x, double& s, double& c) {
+    const crmath::SinCos r = crmath::sincos(x);
+    s = r.s;
+    c = r.c;
+}
 CMPMC_HD double m_exp(double x) { return crmath::exp(x); }
 CMPMC_HD double m_pow(double x, double y) { return crmath::pow(x, y); }
 CMPMC_HD double m_hypot(double x, double y) { return crmath::hypot(x, y); }
@@ -42,6 +47,10 @@ CMPMC_HD double m_atan2(double y, double x) { return crmath::atan2(y, x); }
 CMPMC_HD double m_log(double x) { return ::log(x); }
 CMPMC_HD double m_sin(double x) { return ::sin(x); }
 CMPMC_HD double m_cos(double x) { return ::cos(x); }
+CMPMC_HD void m_sincos(double x, double& s, double& c) {
+    s = ::sin(x);
+    c = ::cos(x);
+}
 CMPMC_HD double m_exp(double x) { return ::exp(x); }
 CMPMC_HD double m_pow(double x, double y) { return ::pow(x, y); }
 CMPMC_HD double m_hypot(double x, double y) { return ::hypot(x, y); }
@@ -160,7 +169,9 @@ struct Rng {
         const double cos_theta = 2.0 * uniform() - 1.0;
         const double sin_theta = sqrt(dmax(0.0, 1.0 - cos_theta * cos_theta));
         const double phi = kTwoPi * uniform();
-        return v3(sin_theta * m_cos(phi), sin_theta * m_sin(phi), cos_theta);
+        double s, c;
+        m_sincos(phi, s, c);
+        return v3(sin_theta * c, sin_theta * s, cos_theta);
     }
     // rng.hpp:86-96
     CMPMC_HD V3 lambertian_dir(V3 n) {
@@ -169,7 +180,9 @@ struct Rng {
         const double cos_theta = sqrt(dmax(0.0, 1.0 - sin_theta * sin_theta));
         const V3 u = orthogonal_unit(n);
         const V3 v = cross(n, u);
-        return unit(u * (sin_theta * m_cos(phi)) + v * (sin_theta * m_sin(phi)) + n * cos_theta);
+        double s, c;
+        m_sincos(phi, s, c);
+        return unit(u * (sin_theta * c) + v * (sin_theta * s) + n * cos_theta);
     }
 };
 
@@ -392,7 +405,8 @@ struct BHit {
     V3 n_in;
     int surf;
 };
-CMPMC_HD BHit intersect_exit(double radius, double half_z, V3 p, V3 v) {
+// The exit distance and surface; the inward normal is needed only where a step ends there
+CMPMC_HD BHit exit_distance(double radius, double half_z, V3 p, V3 v) {
     double t_min = kInf;
     int surf = 2;
     if (v.z > 1e-15) {
@@ -410,19 +424,22 @@ CMPMC_HD BHit intersect_exit(double radius, double half_z, V3 p, V3 v) {
         const double tr = (-b + sqrt(disc)) / a;
         if (tr >= 0.0 && tr < t_min) { t_min = tr; surf = 2; }
     }
-    t_min = dmax(0.0, t_min);
     BHit h;
-    h.distance = t_min;
+    h.distance = dmax(0.0, t_min);
     h.surf = surf;
-    if (surf == 0) {
-        h.n_in = v3(0.0, 0.0, -1.0);
-    } else if (surf == 1) {
-        h.n_in = v3(0.0, 0.0, 1.0);
-    } else {
-        const V3 hp = p + v * t_min;
-        const double r_xy = m_hypot(hp.x, hp.y);
-        h.n_in = (r_xy > 1e-15) ? v3(-hp.x / r_xy, -hp.y / r_xy, 0.0) : v3(-1.0, 0.0, 0.0);
-    }
+    h.n_in = v3(0.0, 0.0, 0.0);
+    return h;
+}
+// inward normal of surface `surf` at the exit point hp = p + v * distance
+CMPMC_HD V3 exit_normal(int surf, V3 hp) {
+    if (surf == 0) return v3(0.0, 0.0, -1.0);
+    if (surf == 1) return v3(0.0, 0.0, 1.0);
+    const double r_xy = m_hypot(hp.x, hp.y);
+    return (r_xy > 1e-15) ? v3(-hp.x / r_xy, -hp.y / r_xy, 0.0) : v3(-1.0, 0.0, 0.0);
+}
+CMPMC_HD BHit intersect_exit(double radius, double half_z, V3 p, V3 v) {
+    BHit h = exit_distance(radius, half_z, p, v);
+    h.n_in = exit_normal(h.surf, p + v * h.distance);
     return h;
 }
 

@@ -66,8 +66,13 @@ struct Hit {
     int surf, excitation, mode;
 };
 
+// The rare branches of the step loops are out of line (CMPMC_HD_COLD): inlined at every use,
+// the group-velocity map and the samplers made loops that the instruction cache does not
+// hold. They take copies of the generator and the track, so that only the copies have their
+// address taken and the loops keep theirs in registers.
+
 // SimulationEngine::make_track (engine.hpp:171-187)
-CMPMC_HD Track make_track(const Lattice& L, V3 pos, V3 k_dir, int mode, double e, double t, double w) {
+CMPMC_HD_COLD Track make_track(const Lattice& L, V3 pos, V3 k_dir, int mode, double e, double t, double w) {
     const V3 ku = unit(k_dir);
     const Kin kin = map_k_to_vg(L, mode, ku);
     Track r;
@@ -84,7 +89,7 @@ CMPMC_HD Track make_track(const Lattice& L, V3 pos, V3 k_dir, int mode, double e
 }
 
 // SimulationEngine::sample_inward_wavevector (engine.hpp:927-936)
-CMPMC_HD V3 sample_inward(const Lattice& L, int mode, V3 n, Rng& rng) {
+CMPMC_HD_COLD V3 sample_inward_cold(const Lattice& L, int mode, V3 n, Rng& rng) {
     for (int trial = 0; trial < 16; ++trial) {
         const V3 kd = rng.lambertian_dir(n);
         const Kin kin = map_k_to_vg(L, mode, kd);
@@ -92,48 +97,72 @@ CMPMC_HD V3 sample_inward(const Lattice& L, int mode, V3 n, Rng& rng) {
     }
     return n;
 }
+CMPMC_HD V3 sample_inward(const Lattice& L, int mode, V3 n, Rng& rng) {
+    Rng g = rng;
+    const V3 k = sample_inward_cold(L, mode, n, g);
+    rng = g;
+    return k;
+}
+CMPMC_HD_COLD Kin map_k_to_vg_cold(const Lattice& L, int mode, V3 k) { return map_k_to_vg(L, mode, k); }
+
+// KaplanFilm::absorb_quantum; the re-emitted energies in refl[0, n_refl)
+CMPMC_HD_COLD double film_absorb_cold(const Film& f, double e, double* refl, int& n_refl, double* work, Rng& rng,
+                                      bool photon) {
+    KBuf r{refl, 0};
+    const double edep = film_absorb_quantum(f, e, r, work, rng, photon);
+    n_refl = r.n;
+    return edep;
+}
+CMPMC_HD double film_absorb(const Film& f, double e, KBuf& refl, double* work, Rng& rng, bool photon) {
+    Rng g = rng;
+    int n = 0;
+    const double edep = film_absorb_cold(f, e, refl.d, n, work, g, photon);
+    rng = g;
+    refl.n = n;
+    return edep;
+}
 
 CMPMC_HD void set_kin(Track& trk, const Kin& kin) {
     trk.vg = kin.vg_dir;
     trk.vmag = kin.vg_mag;
 }
 
-// SimulationEngine::perform_anharmonic_decay (engine.hpp:938-988)
-template <class C>
-CMPMC_HD void anharmonic_decay(const Lattice& L, Track& trk, C& ctx, EvStats& st, Rng& rng) {
+// SimulationEngine::perform_anharmonic_decay (engine.hpp:938-988): the parent continues in trk,
+// the daughter goes to dtr; true for the two-transverse channel
+CMPMC_HD_COLD bool decay_cold(const Lattice& L, Track& trk, Track& dtr, Rng& rng) {
     const V3 dir1 = trk.k;
     const V3 perp = orthogonal_unit(dir1);
     const double phi = kTwoPi * rng.uniform();
-    const double c_phi = m_cos(phi);
-    const double s_phi = m_sin(phi);
-    if (rng.uniform() < L.fTT_frac) {
-        st.decays_TT++;
-        const double x = sample_cdf(L.cdf_tt, rng);
-        const double th1 = decay_angle_TT(x, L.v_sound, L.v_trans);
-        const double th2 = decay_angle_TT(1.0 - x, L.v_sound, L.v_trans);
-        const V3 k1 = unit(rotate_around(rotate_around(dir1, perp, m_cos(th1), m_sin(th1)), dir1, c_phi, s_phi));
-        const V3 k2 = unit(rotate_around(rotate_around(dir1, perp, m_cos(-th2), m_sin(-th2)), dir1, c_phi, s_phi));
-        const int m1 = sample_transverse_mode(L, rng);
-        const int m2 = sample_transverse_mode(L, rng);
-        ctx.push(make_track(L, trk.pos, k2, m2, (1.0 - x) * trk.E, trk.t, trk.w));
-        trk.E = x * trk.E;
-        trk.mode = m1;
-        trk.k = k1;
-        set_kin(trk, map_k_to_vg(L, m1, k1));
-    } else {
-        st.decays_LT++;
-        const double x = sample_cdf(L.cdf_lt, rng);
-        const double thL = decay_angle_L_to_LT(x, L.v_sound, L.v_trans);
-        const double thT = decay_angle_T_from_LT(x, L.v_sound, L.v_trans);
-        const V3 kL = unit(rotate_around(rotate_around(dir1, perp, m_cos(thL), m_sin(thL)), dir1, c_phi, s_phi));
-        const V3 kT = unit(rotate_around(rotate_around(dir1, perp, m_cos(-thT), m_sin(-thT)), dir1, c_phi, s_phi));
-        const int mT = sample_transverse_mode(L, rng);
-        ctx.push(make_track(L, trk.pos, kT, mT, (1.0 - x) * trk.E, trk.t, trk.w));
-        trk.E = x * trk.E;
-        trk.mode = 0;
-        trk.k = kL;
-        set_kin(trk, map_k_to_vg(L, 0, kL));
-    }
+    double s_phi, c_phi;
+    m_sincos(phi, s_phi, c_phi);
+    const bool tt = rng.uniform() < L.fTT_frac;
+    const double x = sample_cdf(tt ? L.cdf_tt : L.cdf_lt, rng);
+    const double th1 = tt ? decay_angle_TT(x, L.v_sound, L.v_trans) : decay_angle_L_to_LT(x, L.v_sound, L.v_trans);
+    const double th2 =
+        tt ? decay_angle_TT(1.0 - x, L.v_sound, L.v_trans) : decay_angle_T_from_LT(x, L.v_sound, L.v_trans);
+    double s1, c1, s2, c2;
+    m_sincos(th1, s1, c1);
+    m_sincos(-th2, s2, c2);
+    const V3 k1 = unit(rotate_around(rotate_around(dir1, perp, c1, s1), dir1, c_phi, s_phi));
+    const V3 k2 = unit(rotate_around(rotate_around(dir1, perp, c2, s2), dir1, c_phi, s_phi));
+    const int m1 = tt ? sample_transverse_mode(L, rng) : 0;
+    const int m2 = sample_transverse_mode(L, rng);
+    dtr = make_track(L, trk.pos, k2, m2, (1.0 - x) * trk.E, trk.t, trk.w);
+    trk.E = x * trk.E;
+    trk.mode = m1;
+    trk.k = k1;
+    set_kin(trk, map_k_to_vg_cold(L, m1, k1));
+    return tt;
+}
+template <class C>
+CMPMC_HD void anharmonic_decay(const Lattice& L, Track& trk, C& ctx, EvStats& st, Rng& rng) {
+    Track t = trk, d;
+    Rng g = rng;
+    if (decay_cold(L, t, d, g)) st.decays_TT++;
+    else st.decays_LT++;
+    trk = t;
+    rng = g;
+    ctx.push(d);
 }
 
 // SimulationEngine::transport (engine.hpp:403-582). ctx provides
@@ -142,6 +171,8 @@ CMPMC_HD void anharmonic_decay(const Lattice& L, Track& trk, C& ctx, EvStats& st
 template <class C>
 CMPMC_HD void transport_phonons(const Lattice& L, const Detector& D, C& ctx, EvStats& st, Rng& rng) {
     Track trk;
+    // the rates depend on the energy alone, which changes at a decay or a film only
+    double e_rate = -1.0, rate_iso = 0.0, rate_anh = 0.0;
     while (ctx.pop(trk)) {
         for (;;) {
             if (trk.E < D.min_phonon_eV || trk.bounces >= D.max_bounces) {
@@ -160,12 +191,16 @@ CMPMC_HD void transport_phonons(const Lattice& L, const Detector& D, C& ctx, EvS
                 }
             }
             st.total_steps++;
-            const double rate_iso = isotope_rate(L, trk.E);
+            if (trk.E != e_rate) {
+                e_rate = trk.E;
+                rate_iso = isotope_rate(L, e_rate);
+                rate_anh = downconversion_rate(L, 0, e_rate);
+            }
             const double rate_poly = polycrystal_rate(L, trk.vmag);
-            const double rate_down = downconversion_rate(L, trk.mode, trk.E);
+            const double rate_down = (trk.mode == 0) ? rate_anh : 0.0;
             const double rate_tot = rate_iso + rate_poly + rate_down;
             const double d_phys = (rate_tot > 1e-12) ? (-m_log(rng.uniform()) * (trk.vmag / rate_tot)) : kInf;
-            const BHit bh = intersect_exit(D.radius, D.half_z, trk.pos, trk.vg);
+            BHit bh = exit_distance(D.radius, D.half_z, trk.pos, trk.vg);
 
             // new direction drawn after the branches below: 1 isotropic (Rng::isotropic_dir,
             // rng.hpp:78-83), 2 Lambertian about the inward normal with the inward check of
@@ -185,8 +220,8 @@ CMPMC_HD void transport_phonons(const Lattice& L, const Detector& D, C& ctx, EvS
                     new_dir = 1;
                 }
             } else {
-
                 trk.pos = trk.pos + trk.vg * bh.distance;
+                bh.n_in = exit_normal(bh.surf, trk.pos);
                 trk.t += bh.distance / trk.vmag;
                 trk.bounces++;
                 const Surface& s = D.surf[bh.surf];
@@ -200,7 +235,7 @@ CMPMC_HD void transport_phonons(const Lattice& L, const Detector& D, C& ctx, EvS
                                                                         dot(trk.k, bh.n_in))
                                                      : film.film_absorption;
                     if (rng.uniform() < p_enter) {
-                        const double edep = film_absorb_phonon(film, trk.E, ctx.refl, ctx.kwork, rng);
+                        const double edep = film_absorb(film, trk.E, ctx.refl, ctx.kwork, rng, false);
                         if (edep > 0.0) {
                             const double wedep = edep * trk.w;
                             st.sensor_hits++;
@@ -229,7 +264,7 @@ CMPMC_HD void transport_phonons(const Lattice& L, const Detector& D, C& ctx, EvS
                         trk.E = ctx.refl.d[0];
                         trk.mode = sample_dos_mode(L, rng);
                         trk.k = sample_inward(L, trk.mode, bh.n_in, rng);
-                        set_kin(trk, map_k_to_vg(L, trk.mode, trk.k));
+                        set_kin(trk, map_k_to_vg_cold(L, trk.mode, trk.k));
                         continue;
                     }
                 }
@@ -254,13 +289,13 @@ CMPMC_HD void transport_phonons(const Lattice& L, const Detector& D, C& ctx, EvS
                     trk.E = x * trk.E;
                     trk.mode = m1;
                     trk.k = sample_inward(L, m1, bh.n_in, rng);
-                    set_kin(trk, map_k_to_vg(L, m1, trk.k));
+                    set_kin(trk, map_k_to_vg_cold(L, m1, trk.k));
                 } else if (u_refl < split.p_anh + split.p_spec) {
                     V3 k_refl = trk.k - bh.n_in * (2.0 * dot(trk.k, bh.n_in));
-                    Kin kin = map_k_to_vg(L, trk.mode, k_refl);
+                    Kin kin = map_k_to_vg_cold(L, trk.mode, k_refl);
                     if (dot(kin.vg_dir, bh.n_in) <= 1e-6) {
                         k_refl = sample_inward(L, trk.mode, bh.n_in, rng);
-                        kin = map_k_to_vg(L, trk.mode, k_refl);
+                        kin = map_k_to_vg_cold(L, trk.mode, k_refl);
                     }
                     trk.k = k_refl;
                     set_kin(trk, kin);
@@ -290,15 +325,15 @@ CMPMC_HD void transport_phonons(const Lattice& L, const Detector& D, C& ctx, EvS
                         st_ = sqrt(u2);
                         ct_ = sqrt(dmax(0.0, 1.0 - st_ * st_));
                     }
-                    const double cphi = m_cos(phi);
-                    const double sphi = m_sin(phi);
+                    double sphi, cphi;
+                    m_sincos(phi, sphi, cphi);
                     kd = iso ? v3(st_ * cphi, st_ * sphi, ct_)
                              : unit(ou * (st_ * cphi) + ov * (st_ * sphi) + bh.n_in * ct_);
                     kin = map_k_to_vg(L, trk.mode, kd);
                     if (iso || dot(kin.vg_dir, bh.n_in) > 1e-6) break;
                     if (trial == 15) {
                         kd = bh.n_in;
-                        kin = map_k_to_vg(L, trk.mode, kd);
+                        kin = map_k_to_vg_cold(L, trk.mode, kd);
                         break;
                     }
                 }
@@ -323,6 +358,23 @@ CMPMC_HD double ekin_electron(const Lattice& L, int iv, V3 p) {
     return sqrt(norm2(ph) + L.e_cond_mass * L.e_cond_mass) - L.e_cond_mass;
 }
 CMPMC_HD double ekin_hole(const Lattice& L, V3 p) { return sqrt(norm2(p) + L.h_mass * L.h_mass) - L.h_mass; }
+// x / m with inv = 1 / m rounded: two residual corrections of x inv give the correctly rounded
+// quotient (P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990) for quotients in the normal range
+CMPMC_HD double div_by(double x, double m, double inv) {
+    double q = x * inv;
+    q = crmath::fma_rn(crmath::fma_rn(-m, q, x), inv, q);
+    return crmath::fma_rn(crmath::fma_rn(-m, q, x), inv, q);
+}
+// vel_electron with the reciprocals of the mass ratios at hand
+CMPMC_HD V3 vel_electron(const Lattice& L, V3 inv_mass, int iv, V3 p) {
+    const V3 pv = mul(L.valley_rot[iv], p);
+    const V3 ph = v3(pv.x * L.hv_sqrt_inv.x, pv.y * L.hv_sqrt_inv.y, pv.z * L.hv_sqrt_inv.z);
+    const double ek = sqrt(norm2(ph) + L.e_cond_mass * L.e_cond_mass) - L.e_cond_mass;
+    const V3 vv = v3(div_by(pv.x, L.mass_ratio.x, inv_mass.x), div_by(pv.y, L.mass_ratio.y, inv_mass.y),
+                     div_by(pv.z, L.mass_ratio.z, inv_mass.z));
+    return mul_transpose(L.valley_rot[iv], vv) * (kCLight / (ek + L.e_cond_mass));
+}
 CMPMC_HD V3 vel_electron(const Lattice& L, int iv, V3 p) {
     const double ek = ekin_electron(L, iv, p);
     const V3 pv = mul(L.valley_rot[iv], p);
@@ -364,18 +416,14 @@ CMPMC_HD Charge make_charge(const Lattice& L, int type, V3 pos, V3 dir, double e
     return c;
 }
 
-// charge_transport.hpp:82-106
-CMPMC_HD double luke_rate(const Lattice& L, const Charge& c) {
-    double k_mag, k_sound, l0;
-    if (c.type == 1) {
-        k_mag = norm(e2s(L, c.valley, vdiv(c.p, kHbarC)));
-        k_sound = L.k_sound_e;
-        l0 = L.l0_e;
-    } else {
-        k_mag = norm(c.p) / kHbarC;
-        k_sound = L.k_sound_h;
-        l0 = L.l0_h;
-    }
+// |k| of a carrier (charge_transport.hpp:82-91)
+CMPMC_HD double charge_k(const Lattice& L, const Charge& c) {
+    return (c.type == 1) ? norm(e2s(L, c.valley, vdiv(c.p, kHbarC))) : norm(c.p) / kHbarC;
+}
+// charge_transport.hpp:92-106
+CMPMC_HD double luke_rate(const Lattice& L, int type, double k_mag) {
+    const double k_sound = (type == 1) ? L.k_sound_e : L.k_sound_h;
+    const double l0 = (type == 1) ? L.l0_e : L.l0_h;
     if (k_mag <= k_sound) return 0.0;
     const double mach = k_mag / k_sound;
     const double dm = mach - 1.0;
@@ -384,10 +432,9 @@ CMPMC_HD double luke_rate(const Lattice& L, const Charge& c) {
     return (tau > 0.0) ? (1.0 / tau) : 0.0;
 }
 
-// charge_kernels.hpp:329-346 (Quadratic and Linear models)
-CMPMC_HD double intervalley_rate(const Lattice& L, double ek, V3 E) {
-    if (L.n_valleys < 2) return 0.0;
-    if (ek < L.iv_min_energy) return 0.0;
+// the field's intervalley rate of an electron over the threshold (charge_kernels.hpp:329-346,
+// Quadratic and Linear models)
+CMPMC_HD double intervalley_field_rate(const Lattice& L, V3 E) {
     if (L.iv_model == 0) {
         const double e0 = L.iv_quad_field;
         return L.iv_quad_rate * m_pow(e0 * e0 + norm2(E), 0.5 * L.iv_quad_power);
@@ -395,21 +442,26 @@ CMPMC_HD double intervalley_rate(const Lattice& L, double ek, V3 E) {
     const double e_vcm = norm(E) * 0.01;
     return L.iv_lin_rate0 + L.iv_lin_rate1 * m_pow(e_vcm, L.iv_lin_power);
 }
-CMPMC_HD double mfp_rate(double v, double mfp) { return (mfp > 0.0 && mfp < 1e20) ? (v / mfp) : 0.0; }
+CMPMC_HD bool mfp_open(double mfp) { return mfp > 0.0 && mfp < 1e20; }
+CMPMC_HD double mfp_rate(double v, double mfp) { return mfp_open(mfp) ? (v / mfp) : 0.0; }
 
 struct Rates {
     double luke, iv, trap, ion_e, ion_h, tot;
 };
-// SimulationEngine::charge_rates (engine.hpp:876-886)
-CMPMC_HD Rates charge_rates(const Lattice& L, const Charge& c, V3 E) {
-    const double v = norm(c.type == 1 ? vel_electron(L, c.valley, c.p) : vel_hole(L, c.p));
+// SimulationEngine::charge_rates (engine.hpp:876-886) of a carrier with |k| = k_mag and the
+// intervalley rate iv; the velocity is needed only where a trapping channel is open
+CMPMC_HD Rates charge_rates(const Lattice& L, const Charge& c, double k_mag, double iv, bool traps) {
     Rates r;
-    r.luke = luke_rate(L, c);
-    r.iv = (c.type == 1) ? intervalley_rate(L, c.ekin, E) : 0.0;
-    const bool e = (c.type == 1);
-    r.trap = mfp_rate(v, e ? L.e_trap_mfp : L.h_trap_mfp);
-    r.ion_e = mfp_rate(v, e ? L.e_ion_d0_mfp : L.h_ion_d_mfp);
-    r.ion_h = mfp_rate(v, e ? L.e_ion_a_mfp : L.h_ion_a0_mfp);
+    r.luke = luke_rate(L, c.type, k_mag);
+    r.iv = iv;
+    r.trap = r.ion_e = r.ion_h = 0.0;
+    if (traps) {
+        const double v = norm(c.type == 1 ? vel_electron(L, c.valley, c.p) : vel_hole(L, c.p));
+        const bool e = (c.type == 1);
+        r.trap = mfp_rate(v, e ? L.e_trap_mfp : L.h_trap_mfp);
+        r.ion_e = mfp_rate(v, e ? L.e_ion_d0_mfp : L.h_ion_d_mfp);
+        r.ion_h = mfp_rate(v, e ? L.e_ion_a_mfp : L.h_ion_a0_mfp);
+    }
     r.tot = r.luke + r.iv + r.trap + r.ion_e + r.ion_h;
     return r;
 }
@@ -443,7 +495,9 @@ CMPMC_HD LukeEmit emit_luke(const Lattice& L, Charge& c, Rng& rng) {
     const double q = 2.0 * (k_mag * cos_th - k_sound);
     if (q <= 0.0) return none;
     const V3 perp = orthogonal_unit(k_dir);
-    const V3 q_vec = rotate_around(rotate_around(k_dir * q, perp, cos_th, sin_th), k_dir, m_cos(phi), m_sin(phi));
+    double s_phi, c_phi;
+    m_sincos(phi, s_phi, c_phi);
+    const V3 q_vec = rotate_around(rotate_around(k_dir * q, perp, cos_th, sin_th), k_dir, c_phi, s_phi);
     const V3 k_recoil = k_trk - q_vec;
     const double e_ph = norm(q_vec) * L.v_sound * kHbar;
     if (e_ph >= c.ekin || e_ph <= 0.0) return none;
@@ -556,7 +610,7 @@ CMPMC_HD double electrode_film_release(const Lattice& L, const Detector& D, cons
     const V3 p0 = pos + n_in * 1e-11;
     double absorbed = 0.0, emitted = 0.0;
     for (int i = 0; i < n; ++i) {
-        absorbed += film_absorb_quantum(film, q, ctx.refl, ctx.kwork, rng, true);
+        absorbed += film_absorb(film, q, ctx.refl, ctx.kwork, rng, true);
         for (int k = 0; k < ctx.refl.n; ++k) {
             const int m = sample_dos_mode(L, rng);
             const V3 kd = sample_inward(L, m, n_in, rng);
@@ -576,23 +630,59 @@ CMPMC_HD void transport_charges(const Lattice& L, const Detector& D, C& ctx, EvS
     const double e_gap = L.bandgap;
     const double luke_prob = dclamp(D.luke_sample_fraction, 0.0, 1.0);
     const double luke_wt_mult = (luke_prob > 0.0) ? (1.0 / luke_prob) : 0.0;
+    const bool second = (D.charge_stepping == 1);
+    const double dk_frac = second ? D.charge_sampling_dk_frac : D.charge_max_dk_frac;
+    const bool traps = mfp_open(L.e_trap_mfp) || mfp_open(L.h_trap_mfp) || mfp_open(L.e_ion_d0_mfp) ||
+                       mfp_open(L.e_ion_a_mfp) || mfp_open(L.h_ion_d_mfp) || mfp_open(L.h_ion_a0_mfp);
+    const V3 inv_mass = v3(1.0 / L.mass_ratio.x, 1.0 / L.mass_ratio.y, 1.0 / L.mass_ratio.z);
+    // |k| surely below / surely above the intervalley threshold: the energy is a difference of
+    // numbers of the size of the mass, so the band holds its rounding too
+    const double slack = 1e-6 * L.iv_min_energy + 1e-14 * L.e_cond_mass;
+    const double e_lo = L.iv_min_energy - slack, e_hi = L.iv_min_energy + slack;
+    const double k_lo = (e_lo > 0.0) ? sqrt(e_lo * e_lo + 2.0 * e_lo * L.e_cond_mass) / kHbarC : -1.0;
+    const double k_hi = (e_hi > 0.0) ? sqrt(e_hi * e_hi + 2.0 * e_hi * L.e_cond_mass) / kHbarC : -1.0;
+    const double edge = 1e-6 * (D.radius + D.half_z);
+    // of the last field value: |dk/dt| of a unit mass factor, and the intervalley rate once needed
+    V3 E_last = v3(kInf, 0.0, 0.0);
+    double dk_field = 0.0, iv_field = 0.0;
+    bool iv_known = false;
     Charge c;
     while (ctx.pop_charge(c)) {
+        // c.ekin follows c.p only where it is read: a step without an event leaves it, and the next
+        // one compares |k| with the intervalley threshold instead
+        bool ek_known = true;
         const double q_sign = (c.type == 1) ? -1.0 : +1.0;
         for (uint32_t step = 0; step < 20000000u; ++step) {
             st.charge_steps++;
             const V3 E = ctx.field(c.pos, c);
-            const bool second = (D.charge_stepping == 1);
-            const double dk_frac = second ? D.charge_sampling_dk_frac : D.charge_max_dk_frac;
-            const Rates R0 = charge_rates(L, c, E);
+            if (!(E.x == E_last.x && E.y == E_last.y && E.z == E_last.z)) {
+                E_last = E;
+                dk_field = norm(E) * kCLight / kHbarC;
+                iv_known = false;
+            }
+            const bool is_e = (c.type == 1);
+            auto iv_of = [&](bool below) {
+                if (!is_e || L.n_valleys < 2 || below) return 0.0;
+                if (!iv_known) {
+                    iv_field = intervalley_field_rate(L, E);
+                    iv_known = true;
+                }
+                return iv_field;
+            };
+            const double k_now = charge_k(L, c);
+            bool below = false;
+            if (is_e)
+                below = ek_known ? c.ekin < L.iv_min_energy
+                                 : (k_now < k_lo || k_now > k_hi)
+                                       ? k_now < k_lo
+                                       : ekin_electron(L, c.valley, c.p) < L.iv_min_energy;
+            const Rates R0 = charge_rates(L, c, k_now, iv_of(below), traps);
             double r_luke = R0.luke, r_iv = R0.iv, r_trap = R0.trap, r_ion_e = R0.ion_e, r_ion_h = R0.ion_h;
             double r_tot = R0.tot;
             double dt_max = D.charge_dt_cap_s;
             if (dk_frac > 0.0) {
-                const bool is_e = (c.type == 1);
                 const double ks = is_e ? L.k_sound_e : L.k_sound_h;
-                const double k_now = is_e ? norm(e2s(L, c.valley, vdiv(c.p, kHbarC))) : norm(c.p) / kHbarC;
-                const double dk_rate = norm(E) * kCLight / kHbarC * (is_e ? hv_max_scale(L) : 1.0);
+                const double dk_rate = dk_field * (is_e ? hv_max_scale(L) : 1.0);
                 if (dk_rate > 0.0) dt_max = dmin(dt_max, dk_frac * dmax(ks, k_now) / dk_rate);
             }
             double dt_phys;
@@ -602,7 +692,7 @@ CMPMC_HD void transport_charges(const Lattice& L, const Detector& D, C& ctx, EvS
                 trial.p = trial.p + E * (q_sign * kCLight * dt_max);
                 trial.ekin = charge_ekin(L, trial);
                 const double a0 = R0.tot;
-                const double a1 = (charge_rates(L, trial, E).tot - a0) / dt_max;
+                const double a1 = (charge_rates(L, trial, charge_k(L, trial), iv_of(trial.ekin < L.iv_min_energy), traps).tot - a0) / dt_max;
                 const double lnu = m_log(rng.uniform());
                 if (fabs(a1) * dt_max <= 1e-9 * dmax(a0, 1e-300)) {
                     dt_phys = (a0 > 0.0) ? (-lnu / a0) : kInf;
@@ -617,11 +707,17 @@ CMPMC_HD void transport_charges(const Lattice& L, const Detector& D, C& ctx, EvS
             const double dt = dmin(dt_phys, dt_max);
             const V3 dp = E * (q_sign * kCLight * dt);
             const V3 p_mid = c.p + dp * 0.5;
-            const V3 v_mid = (c.type == 1) ? vel_electron(L, c.valley, p_mid) : vel_hole(L, p_mid);
+            const V3 v_mid = is_e ? vel_electron(L, inv_mass, c.valley, p_mid) : vel_hole(L, p_mid);
             const double v_mid_mag = norm(v_mid);
             const double d_step = v_mid_mag * dt;
 
-            if (v_mid_mag > 1e-6) {
+            // a carrier whose distance to every wall is over twice the step (plus an edge far above
+            // the rounding of the exit point) cannot reach one; anything not finite takes the test
+            const double reach = 2.0 * d_step + edge;
+            const double r_in = D.radius - reach;
+            const bool inside = r_in > 0.0 && fabs(c.pos.z) < D.half_z - reach &&
+                                c.pos.x * c.pos.x + c.pos.y * c.pos.y < r_in * r_in;
+            if (!inside && v_mid_mag > 1e-6) {
                 const V3 v_dir = vdiv(v_mid, v_mid_mag);
                 const BHit bh = intersect_exit(D.radius, D.half_z, c.pos, v_dir);
                 if (bh.distance <= d_step) {
@@ -630,6 +726,7 @@ CMPMC_HD void transport_charges(const Lattice& L, const Detector& D, C& ctx, EvS
                     c.t += dt_b;
                     c.p = c.p + E * (q_sign * kCLight * dt_b);
                     c.ekin = charge_ekin(L, c);
+                    ek_known = true;
                     const Surface& s = D.surf[bh.surf];
                     // electrode mask (engine.hpp:284-289)
                     const int ch_id = (s.n_pads > 0) ? find_channel(s.pads, s.n_pads, c.pos.x, c.pos.y, rng) : -1;
@@ -674,11 +771,11 @@ CMPMC_HD void transport_charges(const Lattice& L, const Detector& D, C& ctx, EvS
             c.pos = c.pos + v_mid * dt;
             c.t += dt;
             c.p = c.p + dp;
-            c.ekin = charge_ekin(L, c);
-
+            ek_known = dt_phys <= dt_max;
             if (dt_phys <= dt_max) {
+                c.ekin = charge_ekin(L, c);
                 if (second) {
-                    const Rates R = charge_rates(L, c, E);
+                    const Rates R = charge_rates(L, c, charge_k(L, c), iv_of(c.ekin < L.iv_min_energy), traps);
                     r_luke = R.luke; r_iv = R.iv; r_trap = R.trap; r_ion_e = R.ion_e; r_ion_h = R.ion_h; r_tot = R.tot;
                     if (r_tot <= 0.0) continue;
                 }

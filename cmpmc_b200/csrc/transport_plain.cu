@@ -123,7 +123,19 @@ struct PlainCtx {
     }
 };
 
-__global__ void __launch_bounds__(128) k_plain_fp64(const Lattice L, const Detector D, const RunArgs a) {
+// An event is one serial stream, so a step's instructions are its latency, and the step loops
+// are larger than the instruction cache: beyond one warp per scheduler the warps wait for
+// instructions first (7 of 12 cycles per issue at 2,000 phonon events). So the step computes
+// nothing that it does not read (exit normals, energies between events, the field's intervalley
+// power at every step), sine and cosine come from one reduction, log and exp have no division,
+// the transcendentals and the rare branches are out of line, and a phonon-only run takes a
+// kernel without the carriers' loop (kCharges). 2,000 phonon events 84 -> 58 ms, 203 mixed
+// events 234 -> 122 ms. Blocks per SM (phonons / mixed, ms): two 68 / 122, three 58 / 137, four
+// 63 / 144, five 67 / 152: more warps pay for phonons, registers without spills for carriers.
+template <bool kCharges>
+__global__ void __launch_bounds__(128, kCharges ? 2 : 3) k_plain_fp64(const __grid_constant__ Lattice L,
+                                                    const __grid_constant__ Detector D,
+                                                    const __grid_constant__ RunArgs a) {
     if (!lane_active(a.lanes)) return;
     const uint64_t slot = lane_slot(a.lanes);
     double refl_buf[kKaplanCap];
@@ -169,7 +181,9 @@ __global__ void __launch_bounds__(128) k_plain_fp64(const Lattice L, const Detec
         for (int k = 0; k < 4; ++k) rng.s[k] = a.rng_state[4 * ev + k];
         EvStats st;
         memset(&st, 0, sizeof(st));
-        if (ctx.n_cinit > 0) transport_charges(L, D, ctx, st, rng);
+        if constexpr (kCharges) {
+            if (ctx.n_cinit > 0) transport_charges(L, D, ctx, st, rng);
+        }
         if (ctx.n_init > 0 || ctx.n_stk > 0) transport_phonons(L, D, ctx, st, rng);
         stats_from_event(st, a.injected[ev], a.ev_stats[ev]);
         a.ev_nhits[ev] = a.keep_hits ? ctx.n_hits : 0;
@@ -183,8 +197,9 @@ __global__ void k_math_check(uint64_t n, const double* __restrict__ x, double* _
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         out[3 * i + 0] = crmath::log(x[i]);
-        out[3 * i + 1] = crmath::sin(x[i]);
-        out[3 * i + 2] = crmath::cos(x[i]);
+        const crmath::SinCos sc = crmath::sincos(x[i]);
+        out[3 * i + 1] = sc.s;
+        out[3 * i + 2] = sc.c;
     }
 }
 
@@ -195,12 +210,14 @@ cudaError_t launch_math_check(uint64_t n, const double* x, double* out) {
 
 cudaError_t launch_plain_fp64(const Lattice& L, const Detector& D, const RunArgs& a, int grid, int block,
                               cudaStream_t s) {
-    k_plain_fp64<<<grid, block, 0, s>>>(L, D, a);
+    if (a.ch_off) k_plain_fp64<true><<<grid, block, 0, s>>>(L, D, a);
+    else k_plain_fp64<false><<<grid, block, 0, s>>>(L, D, a);
     return cudaGetLastError();
 }
 
-cudaError_t plain_fp64_occupancy(int block, int* blocks_per_sm) {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_plain_fp64, block, 0);
+cudaError_t plain_fp64_occupancy(int block, bool charges, int* blocks_per_sm) {
+    if (charges) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_plain_fp64<true>, block, 0);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_plain_fp64<false>, block, 0);
 }
 
 }  // namespace cmpmc_gpu
@@ -292,7 +309,7 @@ struct NoAllocCtx {
 
 // pass 0 counts hits into hit_offsets[ev + 1]; pass 1 writes them at hit_offsets[ev]
 __global__ void __launch_bounds__(kNoAllocThreads)
-    k_plain_fp64_noalloc(const Lattice L, const Detector D, uint64_t n_events, const uint64_t* __restrict__ rng_state,
+    k_plain_fp64_noalloc(const __grid_constant__ Lattice L, const __grid_constant__ Detector D, uint64_t n_events, const uint64_t* __restrict__ rng_state,
                          const double* __restrict__ injected, const uint64_t* __restrict__ ph_off,
                          const cmpmc_phonon_track* __restrict__ ph, cmpmc_sim_stats* __restrict__ ev_stats,
                          uint64_t* __restrict__ hit_offsets, cmpmc_sensor_hit* __restrict__ hits, int pass,
