@@ -93,3 +93,27 @@ def test_carrier_sizes(ge_lattice, n):
     packed = eng.generate(cm.workloads.pair_drift, n, 11)
     opt = cm.RunOptions(seed=11, form="batched_fp32", want_event_stats=True)
     _same(eng.run_packed(packed, opt), dense.run_packed(packed, opt))
+
+
+# one deposit per warp up to 1,184 (two 128-thread blocks on each of 148 SMs), then two
+@pytest.mark.parametrize("n", [1, 1184, 1185, 2369])
+def test_partition_sizes(ge_lattice, n):
+    """Deposits in one call and one by one groups of 37: the same records and final states."""
+    import cmpmc_b200 as cm
+    from cmpmc_b200 import _ffi
+    rng = np.random.default_rng(n)
+    dep = np.zeros(n, dtype=_ffi.DEPOSIT_DTYPE)
+    dep["pos"] = rng.uniform(-0.01, 0.01, (n, 3))
+    dep["edep_eV"] = 10.0 ** rng.uniform(1.0, 4.0, n)
+    dep["is_nuclear_recoil"] = np.arange(n) % 2
+    states = rng.integers(1, 1 << 63, size=(n, 4), dtype=np.uint64)
+    eng = _engine(ge_lattice)
+    opts = cm.PartitionOptions(max_sampled_pairs=16, max_sampled_phonons=8)
+    coff, ch, poff, ph, st = cm.partition_deposits_on_device(eng, dep, states, opts)
+    for lo in range(0, n, max(37, n // 3)):
+        hi = min(n, lo + 37)
+        c2, ch2, p2, ph2, st2 = cm.partition_deposits_on_device(eng, dep[lo:hi], states[lo:hi], opts)
+        assert np.array_equal(coff[lo:hi + 1] - coff[lo], c2) and np.array_equal(poff[lo:hi + 1] - poff[lo], p2)
+        assert ch[int(coff[lo]):int(coff[hi])].tobytes() == ch2.tobytes()
+        assert ph[int(poff[lo]):int(poff[hi])].tobytes() == ph2.tobytes()
+        assert np.array_equal(st[lo:hi], st2)
