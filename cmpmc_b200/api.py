@@ -1101,15 +1101,15 @@ class SimulationEngine:
         out = _ffi.RunOutC()
         _check(self._lib.cmpmc_gpu_run_events(h, C.byref(d), C.byref(out)), h)
         nh = int(out.n_hits)
-        hits = np.zeros(nh, dtype=_ffi.HIT_DTYPE)
+        hits = np.empty(nh, dtype=_ffi.HIT_DTYPE)
         if nh:
-            C.memmove(hits.ctypes.data, out.hits, nh * _ffi.HIT_DTYPE.itemsize)
+            _check(self._lib.cmpmc_copy_out(hits.ctypes.data, out.hits, nh * _ffi.HIT_DTYPE.itemsize))
         offs = np.zeros(n + 1, dtype=np.uint64)
         C.memmove(offs.ctypes.data, out.hit_offsets, (n + 1) * 8)
         evst = None
         if options.want_event_stats and n:
-            evst = np.zeros(n, dtype=_ffi.STATS_DTYPE)
-            C.memmove(evst.ctypes.data, out.event_stats, n * _ffi.STATS_DTYPE.itemsize)
+            evst = np.empty(n, dtype=_ffi.STATS_DTYPE)
+            _check(self._lib.cmpmc_copy_out(evst.ctypes.data, out.event_stats, n * _ffi.STATS_DTYPE.itemsize))
         stats = SimStats(np.frombuffer(bytes(out.stats), dtype=_ffi.STATS_DTYPE)[0])
         return RunResult(stats=stats, hits=hits, hit_offsets=offs, threads_used=1, kernel_ms=out.kernel_ms,
                          device_ms=out.total_ms, kernel_launches=int(out.kernel_launches), event_stats=evst)

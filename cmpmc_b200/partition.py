@@ -261,8 +261,9 @@ def partition_deposits_on_device(engine, deposits, rng_state, opts: Optional[Par
     t_ph = torch.zeros(max(1, nph.value) * 128, dtype=torch.uint8, device=dev)
     _check(lib.cmpmc_gpu_partition_deposits(*args, t_ch.data_ptr(), nc.value, t_ph.data_ptr(), nph.value,
                                             C.byref(nc), C.byref(nph)), h)
-    ch = t_ch.cpu().numpy().view(_ffi.CHARGE_DTYPE)[:nc.value].copy()
-    ph = t_ph.cpu().numpy().view(_ffi.PHONON_DTYPE)[:nph.value].copy()
+    # .cpu() made arrays of their own, of the exact size: no further copy
+    ch = t_ch.cpu().numpy().view(_ffi.CHARGE_DTYPE)[:nc.value]
+    ph = t_ph.cpu().numpy().view(_ffi.PHONON_DTYPE)[:nph.value]
     return (t_coff.cpu().numpy().view(np.uint64), ch, t_poff.cpu().numpy().view(np.uint64), ph,
             t_rng.cpu().numpy().view(np.uint64).reshape(n, 4))
 

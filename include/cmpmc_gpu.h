@@ -693,6 +693,10 @@ typedef struct cmpmc_adjoint_out {
 
 int cmpmc_gpu_adjoint(cmpmc_gpu_ctx* ctx, const cmpmc_adjoint_desc* desc, cmpmc_adjoint_out* out);
 
+/* Copies `bytes` of a result out of the library's buffers into the caller's memory, on several
+ * host threads when it is large. Host memory only. */
+int cmpmc_copy_out(void* dst, const void* src, size_t bytes);
+
 /* Correctly rounded log / sin / cos of the device transport (crmath), evaluated on the
  * host; the device computes bit-identical values. */
 double cmpmc_cr_log(double x);
