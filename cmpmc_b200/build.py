@@ -56,7 +56,7 @@ def _nvcc() -> str:
 
 
 def _headers() -> list[str]:
-    hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".hpp", ".h"))]
+    hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".hpp", ".h", ".inl"))]
     hs.append(os.path.join(INCLUDE, "cmpmc_gpu.h"))
     return hs
 

@@ -102,7 +102,7 @@ struct cmpmc_gpu_ctx {
     DevBuf pads[3];                                     // electrode masks of the three surfaces
     DevBuf lut[3];                                      // Kaplan surrogate tables of the films
     bool lut_ready = false;
-    DevBuf queue, resume_a, resume_b, ccounters, carrier_event, cursor;  // batched charge form
+    DevBuf queue, resume_a, resume_b, ccounters, carrier_event, carrier_order, cursor;  // batched charge form
     DevBuf rel;                                         // batched charge release records
     DevBuf part_plans, part_counts;                     // device partition: plans, per-deposit counts
     DevBuf film_a, queue_b;                             // wavefront split: film entries, second phonon queue
@@ -372,6 +372,12 @@ int run_charges_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a,
     if (n_ph) CK(ctx->unit_event.ensure(n_ph * 4), "alloc unit map");
     CK(launch_carrier_event(a.ch_off, n, ctx->carrier_event.as<uint32_t>(), s), "carrier map");
     ++launches;
+    if (charges_wait(ctx->L, sp_ch.lanes)) {
+        if (n_ch >= (1ull << 32)) return fail(ctx, CMPMC_ERR_INVALID, "too many carriers in one call");
+        CK(ctx->carrier_order.ensure(carrier_order_bytes(n_ch)), "alloc carrier order");
+        CK(launch_carrier_order(ctx->L, ctx->D, a.ch, n_ch, ctx->carrier_order.as<uint32_t>(), s, &launches),
+           "carrier order");
+    }
     if (n_ph) {
         CK(launch_unit_event(a.ph_off, n, ctx->unit_event.as<uint32_t>(), s), "unit map");
         ++launches;
@@ -388,6 +394,7 @@ int run_charges_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a,
     std::memset(&ca, 0, sizeof(ca));
     ca.n_carriers = n_ch;
     ca.carrier_event = ctx->carrier_event.as<uint32_t>();
+    ca.order = ctx->carrier_order.as<uint32_t>();
     ca.carrier_seed = mix64(d->seed ^ 0x2545f4914f6cdd1dULL);
     ca.q_tail = &cc->q_tail;
     ca.resume_next = &cc->resume_next;
@@ -1067,7 +1074,7 @@ void cmpmc_gpu_destroy(cmpmc_gpu_ctx* ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (DevBuf* b : {&ctx->kin, &ctx->film_a, &ctx->queue_b, &ctx->rel, &ctx->part_plans, &ctx->part_counts, &ctx->lut[0], &ctx->lut[1], &ctx->lut[2], &ctx->pads[0], &ctx->pads[1], &ctx->pads[2], &ctx->tables, &ctx->mesh, &ctx->mesh32, &ctx->mesh2, &ctx->mesh2_32, &ctx->queue, &ctx->resume_a, &ctx->resume_b,
-                      &ctx->ccounters, &ctx->carrier_event, &ctx->cursor, &ctx->in_rng, &ctx->in_inj, &ctx->in_phoff, &ctx->in_ph, &ctx->in_choff,
+                      &ctx->ccounters, &ctx->carrier_event, &ctx->carrier_order, &ctx->cursor, &ctx->in_rng, &ctx->in_inj, &ctx->in_phoff, &ctx->in_ph, &ctx->in_choff,
                       &ctx->in_ch, &ctx->stack, &ctx->cstack, &ctx->hit_stage, &ctx->hit_key, &ctx->counters,
                       &ctx->ev_stats, &ctx->ev_nhits, &ctx->offsets, &ctx->hits_out, &ctx->total,
                       &ctx->unit_event, &ctx->ev_offsets, &ctx->ev_stats2, &ctx->partials, &ctx->adj_prim,

@@ -149,6 +149,7 @@ struct ReleaseRec {
 struct ChargeArgs {
     uint64_t n_carriers;              // initial carriers (RunArgs::ch)
     const uint32_t* carrier_event;    // [n_carriers]
+    const uint32_t* order;            // [n_carriers] the order in which they start (waiting form)
     uint64_t carrier_seed;            // substream seed of the carriers
     QPhonon* queue;
     uint64_t q_cap;
@@ -280,6 +281,12 @@ cudaError_t launch_math_check(uint64_t n, const double* x, double* out);
 // phonon kernel over the queue entries; both add to per-event sinks
 cudaError_t launch_charges_fp32(const Lattice& L, const float* cdf_f, const Detector& D, const RunArgs& a,
                                 const ChargeArgs& c, int grid, int block, cudaStream_t s);
+// launch_charges_fp32 takes the form in which event draws wait (ChargeArgs::order must be set)
+bool charges_wait(const Lattice& L, uint32_t lanes);
+// the order in which the n (> 0, < 2^32) carriers start, into order[n] (carrier_order_bytes(n) bytes)
+cudaError_t launch_carrier_order(const Lattice& L, const Detector& D, const cmpmc_charge_track* ch, uint64_t n,
+                                 uint32_t* order, cudaStream_t s, int* launches);
+size_t carrier_order_bytes(uint64_t n);
 cudaError_t charges_fp32_occupancy(int block, int* blocks_per_sm);
 // Exclusive scan of n counts into offsets[0..n] (single block)
 cudaError_t launch_scan_u64(const uint64_t* counts, uint64_t n, uint64_t* offsets, cudaStream_t s);

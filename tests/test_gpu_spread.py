@@ -85,7 +85,8 @@ def test_thread_per_unit_sizes(ge_lattice, form, n):
     _same(a, b)
 
 
-@pytest.mark.parametrize("n", [1, 75, 1481])
+# 518 and 519 events: seven and eight carriers per packed warp, where event draws begin to wait
+@pytest.mark.parametrize("n", [1, 75, 518, 519, 1481])
 def test_carrier_sizes(ge_lattice, n):
     import cmpmc_b200 as cm
     eng, dense = _engine(ge_lattice, drift=True), _engine(ge_lattice, drift=True)
@@ -117,3 +118,27 @@ def test_partition_sizes(ge_lattice, n):
         assert ch[int(coff[lo]):int(coff[hi])].tobytes() == ch2.tobytes()
         assert ph[int(poff[lo]):int(poff[hi])].tobytes() == ph2.tobytes()
         assert np.array_equal(st[lo:hi], st2)
+
+
+# the waiting form (packed: nine carriers per warp) against the other with Luke phonons tracked, a
+# queue that parks carriers, reflecting walls, a mesh field (carriers ordered by type alone) and
+# second-order stepping
+@pytest.mark.parametrize("case", ["queue", "walls", "mesh", "leman"])
+def test_waiting_charges(ge_lattice, case):
+    import cmpmc_b200 as cm
+    from tests.helpers import axisym_mesh
+    det = cm.DetectorModel()
+    det.e_field = cm.UniformElectricField.from_bias(2.0, 2.54 * cm.units.cm)
+    det.luke_sample_fraction = 0.002 if case == "queue" else 0.0
+    if case == "walls":
+        for s in det.surfaces:
+            s.prob_charge_abs, s.prob_charge_spec = 0.5, 0.5
+    elif case == "mesh":
+        det.mesh_field_2d = axisym_mesh(det)
+    elif case == "leman":
+        det.charge_stepping = 1
+    eng, packed_eng = cm.SimulationEngine(ge_lattice, det), cm.SimulationEngine(ge_lattice, det)
+    packed_eng.configure(threads_per_block=32, blocks_per_sm=1, queue_capacity=8192 if case == "queue" else 0)
+    ev = eng.generate(cm.workloads.pair_drift, 620, 23)
+    opt = cm.RunOptions(seed=23, form="batched_fp32", want_event_stats=True)
+    _same(eng.run_packed(ev, opt), packed_eng.run_packed(ev, opt))
