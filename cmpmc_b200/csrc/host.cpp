@@ -97,6 +97,7 @@ Pad pad_view(const cmpmc_electrode_pad& p) {
     o.phi_min = p.phi_min;
     o.phi_max = p.phi_max;
     o.fill = p.fill_fraction;
+    pad_edges(o);
     return o;
 }
 
