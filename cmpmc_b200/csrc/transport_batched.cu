@@ -575,16 +575,27 @@ __device__ __forceinline__ void batched_loop(const FLat& L, const Detector& D, c
                 }
             }
             if (enter) {
+                // the entry step in line: most entries end in it, and each was a call with the
+                // generator and the energies passed through local memory (500 inline events
+                // 86.6 -> 78.3 ms, adjoint of 200 events 113 -> 106 ms)
                 int n_refl = 0;
-                double edep;
-                R128 g_c = g;
-                if constexpr (kSur) {
-                    edep = s.lut_abs ? surrogate_call(&s, trk.E, refl_buf, &n_refl, kwork, &g_c)
-                                     : kaplan_call(&s.film, trk.E, refl_buf, &n_refl, kwork, &g_c);
+                double edep = 0.0;
+                const int film = film_quick<kSur>(&s.film, trk.E, &g);
+                if (film == kFilmAbsorbed) {
+                    edep = trk.E;
+                } else if (film == kFilmReemit) {
+                    n_refl = 1;
+                    refl_buf[0] = trk.E;
                 } else {
-                    edep = kaplan_call(&s.film, trk.E, refl_buf, &n_refl, kwork, &g_c);
+                    R128 g_c = g;
+                    if constexpr (kSur) {
+                        edep = s.lut_abs ? surrogate_call(&s, trk.E, refl_buf, &n_refl, kwork, &g_c)
+                                         : kaplan_call(&s.film, trk.E, refl_buf, &n_refl, kwork, &g_c);
+                    } else {
+                        edep = kaplan_cascade_call(&s.film, trk.E, refl_buf, &n_refl, kwork, &g_c);
+                    }
+                    g = g_c;
                 }
-                g = g_c;
                 if (edep > 0.0) {
                     const double wedep = edep * trk.w;
                     ++st.hits();
