@@ -12,8 +12,8 @@
 // channel is open, no kinetic energy (the intervalley threshold is decided by |k|), and no
 // exit point for a carrier far from every wall. 4,000 carriers 101 -> 66 ms, 100,000 carriers
 // 182 -> 134 ms, the carriers and phonons of 64 light recoils 117 -> 88 ms.
-// (128, 5): 96 registers, five blocks per SM (pair drift of 200,000 events 467 -> 431 ms
-// against (128, 4) at 104 registers; (128, 6) at 80 registers 432 ms)
+// (128, 5): 96 registers, five blocks per SM (with the step as it was, pair drift of 200,000
+// events 467 -> 431 ms against (128, 4) at 104 registers; (128, 6) at 80 registers 432 ms)
 __global__ void __launch_bounds__(128, 5) CHARGE_KERNEL(const __grid_constant__ FCLat Lp,
                                                          const __grid_constant__ FCDet D,
                                                          const __grid_constant__ RunArgs a,
