@@ -1623,6 +1623,7 @@ struct SmPoolArgs {
 
 struct SmShared {
     uint32_t r_head, r_tail, r_pub;  // ring: consumable [r_head, r_pub), appended at r_tail
+    uint32_t r_floor;                // r_head at the start of the phase: ring slots below it are free
     uint32_t f_tail, f_next;         // film buffer: records [0, f_tail), next to run
     uint32_t input_left;             // the batch still has primaries
     uint32_t n_dry;                  // warps of this phase that ran out of work
@@ -2220,7 +2221,7 @@ __global__ void __launch_bounds__(P::kThreads, 1) k_sm_pool(const __grid_constan
     const uint32_t ring_mask = p.ring_cap - 1;
     if constexpr (P::kStage) stage_surf_hot(L, D, s_hot);  // FP32 policy (the FP64 step reads D)
     if (threadIdx.x == 0) {
-        sh.r_head = sh.r_tail = sh.r_pub = 0;
+        sh.r_head = sh.r_tail = sh.r_pub = sh.r_floor = 0;
         sh.f_tail = sh.f_next = 0;
         sh.input_left = 1;
         sh.n_dry = 0;
@@ -2246,7 +2247,10 @@ __global__ void __launch_bounds__(P::kThreads, 1) k_sm_pool(const __grid_constan
     unsigned err = 0;
     for (;;) {
         // ---- transport phase --------------------------------------------------------
-        const uint32_t r_floor = vsh->r_head;  // ring slots below it are free
+        // the boundary's copy of the head: r_head itself moves as soon as the first warp claims, past
+        // entries that have not been read yet and, with claims past the published entries, past the
+        // tail, where an append would count as an overflow
+        const uint32_t r_floor = vsh->r_floor;
         const uint32_t r_pub = vsh->r_pub;
         // entries a warp claims at a time: few waiting entries are spread over the warps
         const uint32_t r_share = (r_pub - r_floor + SmShape<P::kThreads>::kWarps - 1) / SmShape<P::kThreads>::kWarps;
@@ -2339,6 +2343,7 @@ __global__ void __launch_bounds__(P::kThreads, 1) k_sm_pool(const __grid_constan
         // ---- boundary: publish what the phases appended ---------------------------------
         if (threadIdx.x == 0) {
             if (sh.r_head > sh.r_pub) sh.r_head = sh.r_pub;  // claims past the published entries were void
+            sh.r_floor = sh.r_head;
             sh.r_pub = sh.r_tail;
             sh.f_tail = 0;
             sh.f_next = 0;
