@@ -254,11 +254,16 @@ def partition_deposits_on_device(engine, deposits, rng_state, opts: Optional[Par
     o = (opts or PartitionOptions()).to_c()
     nc, nph = C.c_uint64(0), C.c_uint64(0)
     args = (h, t_dep.data_ptr(), n, C.byref(o), t_rng.data_ptr(), t_coff.data_ptr(), t_poff.data_ptr())
+    # the library writes on the context's own stream: torch's zero fills, and whatever the caller
+    # queued on its stream that still uses the memory, come first
+    stream = torch.cuda.current_stream(torch.device(dev))
+    stream.synchronize()
     status = lib.cmpmc_gpu_partition_deposits(*args, None, 0, None, 0, C.byref(nc), C.byref(nph))
     if status not in (0, 4):
         _check(status, h)
     t_ch = torch.zeros(max(1, nc.value) * 128, dtype=torch.uint8, device=dev)
     t_ph = torch.zeros(max(1, nph.value) * 128, dtype=torch.uint8, device=dev)
+    stream.synchronize()
     _check(lib.cmpmc_gpu_partition_deposits(*args, t_ch.data_ptr(), nc.value, t_ph.data_ptr(), nph.value,
                                             C.byref(nc), C.byref(nph)), h)
     # .cpu() made arrays of their own, of the exact size: no further copy
