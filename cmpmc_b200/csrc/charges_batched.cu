@@ -368,6 +368,7 @@ __global__ void k_carrier_event(const uint64_t* __restrict__ ch_off, uint64_t n_
 // Each carrier owns its substream, so the order changes no carrier; it is free within a key.
 constexpr int kOrderBins = 64;
 constexpr int kOrderKeys = 2 * kOrderBins;
+static_assert(kOrderKeys <= 256, "a key is kept in one byte");
 
 __device__ __forceinline__ int order_key(const FCDet& D, const cmpmc_charge_track& c) {
     const bool e = c.type == 1;
@@ -382,16 +383,21 @@ __device__ __forceinline__ int order_key(const FCDet& D, const cmpmc_charge_trac
     return (e ? 0 : kOrderBins) + bin;
 }
 
-// bins[k]: carriers with key k; k_order_start turns the counts into first places
+// bins[k]: carriers with key k; k_order_start turns the counts into first places. The key is
+// computed once and kept (one byte a carrier): were the second kernel to round a distance on the
+// edge of a bin the other way, one place of the order would be written twice and one never.
 __global__ void __launch_bounds__(256) k_order_count(const __grid_constant__ FCDet D,
                                                      const cmpmc_charge_track* __restrict__ ch, uint64_t n,
-                                                     uint32_t* __restrict__ bins) {
+                                                     uint32_t* __restrict__ bins, uint8_t* __restrict__ keys) {
     __shared__ uint32_t cnt[kOrderKeys];
     if (threadIdx.x < kOrderKeys) cnt[threadIdx.x] = 0;
     __syncthreads();
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<uint64_t>(gridDim.x) * blockDim.x)
-        atomicAdd(&cnt[order_key(D, ch[i])], 1u);
+         i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        const int key = order_key(D, ch[i]);
+        keys[i] = static_cast<uint8_t>(key);
+        atomicAdd(&cnt[key], 1u);
+    }
     __syncthreads();
     if (threadIdx.x < kOrderKeys && cnt[threadIdx.x]) atomicAdd(bins + threadIdx.x, cnt[threadIdx.x]);
 }
@@ -409,12 +415,11 @@ __global__ void __launch_bounds__(kOrderKeys) k_order_start(uint32_t* __restrict
     }
     bins[t] = part[t] - own;
 }
-__global__ void __launch_bounds__(256) k_order_place(const __grid_constant__ FCDet D,
-                                                     const cmpmc_charge_track* __restrict__ ch, uint64_t n,
+__global__ void __launch_bounds__(256) k_order_place(const uint8_t* __restrict__ keys, uint64_t n,
                                                      uint32_t* __restrict__ bins, uint32_t* __restrict__ order) {
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<uint64_t>(gridDim.x) * blockDim.x)
-        order[atomicAdd(bins + order_key(D, ch[i]), 1u)] = static_cast<uint32_t>(i);
+        order[atomicAdd(bins + keys[i], 1u)] = static_cast<uint32_t>(i);
 }
 
 // The release phase of the batched charge form (engine.hpp:302-313, 894-925): one collected
@@ -612,18 +617,20 @@ bool charges_wait(const Lattice& L, uint32_t lanes) {
     return lanes >= kWaitLanes && !traps;
 }
 
-size_t carrier_order_bytes(uint64_t n) { return (n + kOrderKeys) * sizeof(uint32_t); }
+// order[n], bins[kOrderKeys], keys[n]
+size_t carrier_order_bytes(uint64_t n) { return (n + kOrderKeys) * sizeof(uint32_t) + n; }
 
 cudaError_t launch_carrier_order(const Lattice& L, const Detector& D, const cmpmc_charge_track* ch, uint64_t n,
                                  uint32_t* order, cudaStream_t s, int* launches) {
     const FCDet d = make_fcdet(D, D.mesh32, L);
     uint32_t* bins = order + n;
+    uint8_t* keys = reinterpret_cast<uint8_t*>(bins + kOrderKeys);
     const cudaError_t e = cudaMemsetAsync(bins, 0, kOrderKeys * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
     const int grid = static_cast<int>(std::min<uint64_t>((n + 255) / 256, 4 * 148));
-    k_order_count<<<grid, 256, 0, s>>>(d, ch, n, bins);
+    k_order_count<<<grid, 256, 0, s>>>(d, ch, n, bins, keys);
     k_order_start<<<1, kOrderKeys, 0, s>>>(bins);
-    k_order_place<<<grid, 256, 0, s>>>(d, ch, n, bins, order);
+    k_order_place<<<grid, 256, 0, s>>>(keys, n, bins, order);
     *launches += 3;
     return cudaGetLastError();
 }
