@@ -372,8 +372,11 @@ CMPMC_HD DD cos_kernel(DD z) {
 CMPMC_HD bool in_range(double x) { return fabs(x) < 1048576.0; }
 
 // Fast sin / cos of a reduced argument r = rh + rl (|r| <= pi/4 + eps) as unrounded (h, l)
-// with relative error below 2^-64 (sin) and 2^-63 (cos): the leading Taylor terms
-// (r^3/6, r^5/120 and r^2/2, r^4/24) in double-double, the rest in FP64.
+// with relative error below 2^-64 (sin) and 2^-66 (cos): the leading Taylor terms
+// (r^3/6, r^5/120 and r^2/2, r^4/24, r^6/720) in double-double, the rest in FP64. The FP64 tail
+// of the cosine starts at r^8/40320 < 2^-18, so its half a dozen roundings stay below 2^-67 of
+// a value above 0.7; from r^6/720 < 2^-11 on they reached 2^-61.1, over the 2^-62 of the
+// rounding test, and sin and cos were a unit off next to midpoints.
 CMPMC_HD DD sin_fast(DD r) {
     const double rh = r.hi, rl = r.lo;
     const DD z = two_prod(rh, rh);                                   // rh^2 exactly
@@ -402,8 +405,12 @@ CMPMC_HD DD cos_fast(DD r) {
     const DD z = two_prod(rh, rh);
     const double w = z.lo + 2.0 * rh * rl;                            // r^2 = z.hi + w
     const DD zsq = two_prod(z.hi, z.hi);
-    const DD t4 = dd_mul(DD{zsq.hi, zsq.lo + 2.0 * z.hi * w}, DD{CMPMC_CR_INV24_HI, CMPMC_CR_INV24_LO});
     const double zz = z.hi;
+    const DD c6 = dd_tab(CMPMC_CR_TAB(cosc), 3);  // -1/720
+    const DD g = two_prod(zz, c6.hi);
+    const DD k = fast_two_sum(CMPMC_CR_INV24_HI, g.hi);  // 1/24 - r^2/720 = k + kl
+    const double kl = k.lo + (CMPMC_CR_INV24_LO + (g.lo + (zz * c6.lo + w * c6.hi)));
+    const DD t46 = dd_mul(DD{zsq.hi, zsq.lo + 2.0 * zz * w}, DD{k.hi, kl});
     double p = 1.0 / 2432902008176640000.0;
     p = fma_rn(zz, p, -1.0 / 6402373705728000.0);
     p = fma_rn(zz, p, 1.0 / 20922789888000.0);
@@ -411,11 +418,10 @@ CMPMC_HD DD cos_fast(DD r) {
     p = fma_rn(zz, p, 1.0 / 479001600.0);
     p = fma_rn(zz, p, -1.0 / 3628800);
     p = fma_rn(zz, p, 1.0 / 40320);
-    p = fma_rn(zz, p, -1.0 / 720);
-    const double tail6 = zz * zz * zz * p;
-    const DD c = two_sum(1.0, -0.5 * z.hi);
-    const DD c2 = two_sum(c.hi, t4.hi);
-    const double lo = c.lo + c2.lo + t4.lo - 0.5 * w + tail6;
+    const double tail8 = zsq.hi * zsq.hi * p;
+    const DD c = two_sum(1.0, -0.5 * zz);
+    const DD c2 = two_sum(c.hi, t46.hi);
+    const double lo = c.lo + c2.lo + t46.lo - 0.5 * w + tail8;
     return fast_two_sum(c2.hi, lo);
 }
 
