@@ -15,6 +15,7 @@
 
 #include "device.cuh"
 #include "internal.hpp"
+#include "launch_shape.hpp"
 
 using namespace cmpmc_gpu;
 
@@ -290,33 +291,6 @@ void grow_pool(cmpmc_gpu_ctx* ctx, unsigned err) {
         else ctx->pool_ring_cap = std::min<uint32_t>(ctx->pool_ring_cap * 4, 1u << 20);
     }
     if ((err & kErrFilmQueue) && sm_pool(ctx)) ctx->sm_film_cap = std::min<uint32_t>(ctx->sm_film_cap * 2, 1u << 20);
-}
-
-// Launch shape of a thread-per-unit kernel (plain, inline, adjoint and charge kernels). A unit
-// is one serial chain of thousands of steps, and the lanes of a warp that hold units wait for
-// each other's branches, so a batch that cannot fill the chip runs fewer units per warp: as
-// many lanes as it takes to give every resident warp work, never more warps than are resident.
-// `late` (percent) lets that share of the units beyond the resident warps start late on a
-// freed lane instead of adding a lane to every warp: it pays where the lengths of the units
-// differ by several times their mean (plain form: 2,000 events on 1,776 warps take 77 ms on
-// one lane and 88 ms on two), not where they are alike (carriers: 115 ms against 99 ms).
-// Measured against 32 lanes of fewer warps: 2,000 plain phonon events 154 -> 77 ms, 203 plain
-// mixed events 507 -> 230 ms, 4,000 carriers 124 -> 99 ms, adjoint of 20,000 primaries
-// 132 -> 111 ms, 50,000 inline primaries 100 -> 97 ms.
-struct Spread {
-    uint64_t grid;   // blocks
-    uint32_t lanes;  // lanes of each warp that take units
-};
-constexpr uint64_t kLatePlain = 25, kLateNone = 0;
-Spread spread_units(uint64_t units, uint64_t max_blocks, int tpb, uint64_t late) {
-    const uint64_t wpb = static_cast<uint64_t>(tpb) / 32;
-    const uint64_t warps = std::max<uint64_t>(1, max_blocks * wpb);
-    const uint64_t room = warps * (100 + late) / 100;
-    units = std::max<uint64_t>(units, 1);
-    Spread r;
-    r.lanes = static_cast<uint32_t>(std::min<uint64_t>(32, (units + room - 1) / room));
-    r.grid = std::max<uint64_t>(1, std::min<uint64_t>(max_blocks, (units + r.lanes * wpb - 1) / (r.lanes * wpb)));
-    return r;
 }
 
 // Device counters of the batched charge form (reset per phase except next_carrier)
@@ -1525,7 +1499,7 @@ int cmpmc_gpu_run_events(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, cmpmc_run_
             bps = std::max(bps, 1);
         }
         const Spread sp = spread_units(units, static_cast<uint64_t>(ctx->num_sms) * bps, ctx->tpb,
-                                       batched ? kLateNone : kLatePlain);
+                                       batched || has_charges ? kLateNone : kLatePhonons);
         const uint64_t grid = sp.grid;
         a.lanes = sp.lanes;
         const uint64_t slots = grid * (ctx->tpb / 32) * sp.lanes;

@@ -79,7 +79,7 @@ struct RunArgs {
     // wavefront split: a track that has taken this many steps in the current phase is parked
     // in `reemit` (next phase) on a substream derived from its own (0: no limit)
     uint32_t phase_steps;
-    // thread-per-unit kernels: lanes of each warp that take units (see spread_lanes)
+    // thread-per-unit kernels: lanes of each warp that take units (spread_units)
     uint32_t lanes;
 };
 
