@@ -113,9 +113,8 @@ struct cmpmc_gpu_ctx {
                                                         // 0 host-driven rounds, 3 SM-phase pool in FP64
     int stage_tables = 1;                               // pool forms: decay CDF tables staged in shared memory
     uint32_t pool_ring_cap = 1024;                      // pending phonons per warp (warp pool)
-    uint32_t sm_ring_cap = 1u << 17;                    // pending phonons per block (SM-phase pool)
-    bool pool_dense = false;                            // a spread small batch overflowed its rings: one block
-                                                        // per 512 units and full rings from then on
+    PoolRing sm_ring;                                   // pending phonons per block (SM-phase pool)
+    PoolShape sm_last{1, 0, 0};                         // the SM-phase pool's last launch
     uint32_t sm_film_cap = 8192;                        // film records per block and phase (SM-phase pool)
     DevBuf pool_ring, pool_film;                        // warp pool: per-warp rings and film buffers
     uint64_t queue_cap = 1ull << 24;                    // Luke-phonon queue entries (64 B each)
@@ -176,8 +175,7 @@ std::vector<uint64_t> graph_key_of(const cmpmc_gpu_ctx* ctx, const cmpmc_run_des
                                static_cast<uint64_t>(d->form), static_cast<uint64_t>(ctx->tpb),
                                static_cast<uint64_t>(ctx->bps), ctx->stack_cap_batched, ctx->hit_cap,
                                static_cast<uint64_t>(ctx->pool), static_cast<uint64_t>(ctx->stage_tables),
-                               ctx->sm_ring_cap, ctx->sm_film_cap, ctx->pool_ring_cap,
-                               static_cast<uint64_t>(ctx->pool_dense)};
+                               ctx->sm_ring.cap, ctx->sm_ring.low, ctx->sm_film_cap, ctx->pool_ring_cap};
     for (const DevBuf* b : {&ctx->stack, &ctx->cstack, &ctx->hit_stage, &ctx->hit_key, &ctx->counters, &ctx->ev_stats,
                             &ctx->ev_nhits, &ctx->offsets, &ctx->hits_out, &ctx->total, &ctx->unit_event,
                             &ctx->ev_offsets, &ctx->ev_stats2, &ctx->partials, &ctx->cursor, &ctx->pool_ring,
@@ -227,15 +225,11 @@ int ensure_surrogate(cmpmc_gpu_ctx* ctx) {
 bool sm_pool(const cmpmc_gpu_ctx* ctx) { return ctx->pool == 1 || ctx->pool == 3; }
 int pool_fp64(const cmpmc_gpu_ctx* ctx) { return ctx->pool == 3 ? 1 : 0; }
 
-// grid of a pool launch over `units` units: one block per SM (SM-phase pool; 512 threads in
-// FP32, 768 in FP64) from the first units on, since a unit's lineage runs on its block alone
-// (a block per 512 units left 108 of 148 SMs without work at 20,300 units: 45 against 26 ms;
-// 100 units 10.8 against 8.5 ms); or the occupancy's 128-thread blocks (warp pool), never
-// more than the units can start
-int pool_grid(cmpmc_gpu_ctx* ctx, uint64_t units, uint64_t* grid) {
+// shape of a pool launch over `units` units: pool_shape (SM-phase pool), or the occupancy's
+// 128-thread blocks (warp pool), never more than the units can start
+int pool_launch_shape(cmpmc_gpu_ctx* ctx, uint64_t units, PoolShape* shape) {
     if (sm_pool(ctx)) {
-        const uint64_t per = ctx->pool_dense ? static_cast<uint64_t>(sm_pool_threads(pool_fp64(ctx))) : 1;
-        *grid = std::max<uint64_t>(1, std::min<uint64_t>(ctx->num_sms, (units + per - 1) / per));
+        *shape = pool_shape(ctx->sm_ring, units, ctx->num_sms, sm_pool_threads(pool_fp64(ctx)));
         return CMPMC_OK;
     }
     int bps = ctx->bps;
@@ -243,51 +237,42 @@ int pool_grid(cmpmc_gpu_ctx* ctx, uint64_t units, uint64_t* grid) {
         CK(pool_fp32_occupancy(128, &bps), "occupancy");
         bps = std::max(bps, 1);
     }
-    *grid = std::max<uint64_t>(1, std::min<uint64_t>(static_cast<uint64_t>(ctx->num_sms) * bps, (units + 127) / 128));
+    const uint64_t grid =
+        std::max<uint64_t>(1, std::min<uint64_t>(static_cast<uint64_t>(ctx->num_sms) * bps, (units + 127) / 128));
+    *shape = PoolShape{grid, ctx->pool_ring_cap, 0};
     return CMPMC_OK;
 }
 
-// ring entries per block of an SM-phase pool launch: the configured capacity is for a block
-// with one unit per thread; blocks that start with fewer units get the same room per unit (a
-// power of two, at least 4,096), so a small batch does not hold a gigabyte of rings
-uint32_t sm_ring_entries(const cmpmc_gpu_ctx* ctx, uint64_t units, uint64_t grid) {
-    if (ctx->pool_dense) return ctx->sm_ring_cap;
-    const uint64_t threads = static_cast<uint64_t>(sm_pool_threads(pool_fp64(ctx)));
-    const uint64_t per_block = (std::max<uint64_t>(units, 1) + grid - 1) / grid;
-    uint32_t cap = std::min<uint32_t>(ctx->sm_ring_cap, 4096);
-    while (cap < ctx->sm_ring_cap && cap / 2 * threads < ctx->sm_ring_cap * per_block) cap *= 2;
-    return cap;
-}
-
-// ring and film buffers for launches of up to `grid` blocks and `units` units
-int ensure_pool_buffers(cmpmc_gpu_ctx* ctx, uint64_t grid, uint64_t units) {
+// ring and film buffers of a launch
+int ensure_pool_buffers(cmpmc_gpu_ctx* ctx, const PoolShape& shape) {
     if (sm_pool(ctx)) {
-        CK(ctx->pool_ring.ensure(grid * sm_ring_entries(ctx, units, grid) * sm_pool_entry_bytes(pool_fp64(ctx))),
-           "alloc block rings");
-        CK(ctx->pool_film.ensure(grid * ctx->sm_film_cap * sm_pool_film_bytes(pool_fp64(ctx))), "alloc film buffers");
+        CK(ctx->pool_ring.ensure(shape.grid * shape.ring * sm_pool_entry_bytes(pool_fp64(ctx))), "alloc block rings");
+        CK(ctx->pool_film.ensure(shape.grid * ctx->sm_film_cap * sm_pool_film_bytes(pool_fp64(ctx))),
+           "alloc film buffers");
     } else {
-        CK(ctx->pool_ring.ensure(grid * 4 * ctx->pool_ring_cap * pool_ring_entry_bytes()), "alloc warp rings");
-        CK(ctx->pool_film.ensure(grid * 4 * pool_film_bytes_per_warp()), "alloc film buffers");
+        CK(ctx->pool_ring.ensure(shape.grid * 4 * shape.ring * pool_ring_entry_bytes()), "alloc warp rings");
+        CK(ctx->pool_film.ensure(shape.grid * 4 * pool_film_bytes_per_warp()), "alloc film buffers");
     }
     return CMPMC_OK;
 }
 
-cudaError_t launch_pool(cmpmc_gpu_ctx* ctx, const RunArgs& a, uint64_t grid, const QPhonon* queue, cudaStream_t s) {
+cudaError_t launch_pool(cmpmc_gpu_ctx* ctx, const RunArgs& a, const PoolShape& shape, const QPhonon* queue,
+                        cudaStream_t s) {
     const uint32_t* ue = ctx->unit_event.as<uint32_t>();
-    if (sm_pool(ctx))
-        return launch_sm_pool_fp32(ctx->L, ctx->cdf_f, ctx->D, a, ctx->pool_ring.p,
-                                   sm_ring_entries(ctx, a.n_events, grid), ctx->pool_film.p,
+    if (sm_pool(ctx)) {
+        ctx->sm_last = shape;
+        return launch_sm_pool_fp32(ctx->L, ctx->cdf_f, ctx->D, a, ctx->pool_ring.p, shape.ring, ctx->pool_film.p,
                                    ctx->sm_film_cap, ue, queue, ctx->stage_tables, pool_fp64(ctx),
-                                   static_cast<int>(grid), s);
-    return launch_pool_fp32(ctx->L, ctx->cdf_f, ctx->D, a, ctx->pool_ring.p, ctx->pool_ring_cap, ctx->pool_film.p, ue,
-                            queue, ctx->stage_tables, static_cast<int>(grid), 128, s);
+                                   static_cast<int>(shape.grid), s);
+    }
+    return launch_pool_fp32(ctx->L, ctx->cdf_f, ctx->D, a, ctx->pool_ring.p, shape.ring, ctx->pool_film.p, ue,
+                            queue, ctx->stage_tables, static_cast<int>(shape.grid), 128, s);
 }
 
-// after an overflow of a pool's ring or film buffer: more room for the rerun
+// after an overflow of a pool's ring or film buffer: more room for the rerun of the last launch
 void grow_pool(cmpmc_gpu_ctx* ctx, unsigned err) {
     if (err & kErrQueue) {
-        if (sm_pool(ctx) && !ctx->pool_dense) ctx->pool_dense = true;
-        else if (sm_pool(ctx)) ctx->sm_ring_cap = std::min<uint32_t>(ctx->sm_ring_cap * 4, 1u << 24);
+        if (sm_pool(ctx)) pool_grow(ctx->sm_ring, ctx->sm_last, sm_pool_threads(pool_fp64(ctx)));
         else ctx->pool_ring_cap = std::min<uint32_t>(ctx->pool_ring_cap * 4, 1u << 20);
     }
     if ((err & kErrFilmQueue) && sm_pool(ctx)) ctx->sm_film_cap = std::min<uint32_t>(ctx->sm_film_cap * 2, 1u << 20);
@@ -387,11 +372,6 @@ int run_charges_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a,
     // film cascades inside; the host-driven rounds (configure_pool 0) split them instead
     const bool pool = d->form == CMPMC_FORM_BATCHED_FP32 && ctx->pool != 0;
     const bool split = d->form == CMPMC_FORM_BATCHED_FP32 && !pool;
-    uint64_t grid_pool = 1;
-    if (pool) {
-        const int st = pool_grid(ctx, ~0ull >> 1, &grid_pool);
-        if (st != CMPMC_OK) return st;
-    }
     int bps_f = ctx->bps;
     if (split && !bps_f) {
         CK(film_fp32_occupancy(tpb, &bps_f), "occupancy");
@@ -469,18 +449,20 @@ int run_charges_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a,
                 ++launches;
             }
         };
-        if (pool) {
-            const int st = ensure_pool_buffers(ctx, grid_pool, ~0ull >> 32);  // the rounds' sizes vary
+        if (pool) {  // the rounds' sizes vary: room for the largest
+            PoolShape full;
+            int st = pool_launch_shape(ctx, ~0ull >> 32, &full);
+            if (st == CMPMC_OK) st = ensure_pool_buffers(ctx, full);
             if (st != CMPMC_OK) return st;
         }
         // one pool launch over `units` units: the primaries (queue == nullptr) or a queue
         auto pool_phase = [&](uint64_t units, const QPhonon* queue) -> int {
             CK(cudaMemsetAsync(&dc->next_work, 0, sizeof(unsigned long long), s), "memset work counter");
             a.n_events = units;
-            uint64_t grid = 1;
-            const int st = pool_grid(ctx, units, &grid);
+            PoolShape shape;
+            const int st = pool_launch_shape(ctx, units, &shape);
             if (st != CMPMC_OK) return st;
-            CK(launch_pool(ctx, a, std::min(grid, grid_pool), queue, s), "pool launch");
+            CK(launch_pool(ctx, a, shape, queue, s), "pool launch");
             ++launches;
             return CMPMC_OK;
         };
@@ -814,10 +796,16 @@ int run_pool_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a, ui
             return CMPMC_OK;
         }
         drop_graph(ctx);  // a ring, film buffer or hit buffer overflowed: rerun eagerly with more room
-        if (hc.err & (kErrQueue | kErrFilmQueue)) grow_pool(ctx, hc.err);
+        if (hc.err & (kErrQueue | kErrFilmQueue)) {
+            PoolShape replayed;  // other launches may have run since the capture
+            const int st = pool_launch_shape(ctx, n_ph, &replayed);
+            if (st != CMPMC_OK) return st;
+            ctx->sm_last = replayed;
+            grow_pool(ctx, hc.err);
+        }
         hc = Counters{};
     }
-    uint64_t grid = 1;
+    PoolShape shape;
     CK(ctx->ev_stats2.ensure(std::max<uint64_t>(n, 1) * sizeof(cmpmc_sim_stats)), "alloc event stats");
     CK(ctx->ev_nhits.ensure(std::max<uint64_t>(n, 1) * 8), "alloc event hit counts");
     CK(ctx->ev_offsets.ensure((n + 1) * 8), "alloc event offsets");
@@ -846,8 +834,17 @@ int run_pool_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a, ui
     for (int attempt = 0;; ++attempt) {
         if (!d->keep_hits) hit_cap = 1;
         {
-            int st = pool_grid(ctx, n_ph, &grid);
-            if (st == CMPMC_OK) st = ensure_pool_buffers(ctx, grid, n_ph);
+            int st = pool_launch_shape(ctx, n_ph, &shape);
+            if (st == CMPMC_OK) st = ensure_pool_buffers(ctx, shape);
+            const uint64_t threads = sm_pool_threads(pool_fp64(ctx));
+            const uint64_t packed = pool_packed_grid(n_ph, ctx->num_sms, threads);
+            if (st != CMPMC_OK && sm_pool(ctx) && shape.grid > packed) {  // no memory for a block on every SM
+                cudaGetLastError();
+                ctx->last_status = CMPMC_OK;
+                ctx->last_error.clear();
+                shape = pool_shape_of(ctx->sm_ring, n_ph, packed, threads);
+                st = ensure_pool_buffers(ctx, shape);
+            }
             if (st != CMPMC_OK) return st;
         }
         CK(ctx->hit_stage.ensure(hit_cap * sizeof(cmpmc_sensor_hit)), "alloc hit staging");
@@ -860,7 +857,7 @@ int run_pool_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a, ui
         CK(cudaMemsetAsync(ctx->counters.p, 0, sizeof(Counters), s), "memset counters");
         CK(cudaEventRecord(ctx->e_k0, s), "event");
         if (n_ph) {
-            CK(launch_pool(ctx, a, grid, nullptr, s), "pool launch");
+            CK(launch_pool(ctx, a, shape, nullptr, s), "pool launch");
             ++launches;
         }
         CK(cudaEventRecord(ctx->e_k1, s), "event");
@@ -903,7 +900,7 @@ int run_pool_batched(cmpmc_gpu_ctx* ctx, const cmpmc_run_desc* d, RunArgs& a, ui
         if (e == cudaSuccess) e = cudaMemsetAsync(ctx->counters.p, 0, sizeof(Counters), s);
         if (e == cudaSuccess) e = launch_unit_event(a.ph_off, n, ctx->unit_event.as<uint32_t>(), s), ++gl;
         if (e == cudaSuccess) e = cudaEventRecordWithFlags(ctx->e_k0, s, cudaEventRecordExternal);
-        if (e == cudaSuccess) e = launch_pool(ctx, ag, grid, nullptr, s), ++gl;
+        if (e == cudaSuccess) e = launch_pool(ctx, ag, shape, nullptr, s), ++gl;
         if (e == cudaSuccess) e = cudaEventRecordWithFlags(ctx->e_k1, s, cudaEventRecordExternal);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(ctx->h_counters.p, ctx->counters.p, sizeof(Counters), cudaMemcpyDeviceToHost, s);
@@ -1226,9 +1223,11 @@ int cmpmc_gpu_configure_pool(cmpmc_gpu_ctx* ctx, int form, uint32_t ring_capacit
         return fail(ctx, CMPMC_ERR_INVALID, "ring capacity: a power of two, at least 64");
     drop_graph(ctx);
     ctx->pool = form;
-    ctx->pool_dense = false;
     if (ring_capacity) {
-        if (form == 1 || form == 3) ctx->sm_ring_cap = std::max<uint32_t>(ring_capacity, 2048);  // a block appends up to 2 x 512 at once
+        if (form == 1 || form == 3) {
+            ctx->sm_ring = PoolRing{};
+            ctx->sm_ring.cap = std::max<uint32_t>(ring_capacity, 2048);  // a block appends up to 2 x 512 at once
+        }
         else ctx->pool_ring_cap = ring_capacity;
     }
     return CMPMC_OK;

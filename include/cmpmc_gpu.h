@@ -534,7 +534,9 @@ int cmpmc_gpu_configure_phases(cmpmc_gpu_ctx* ctx, uint32_t phase_steps);
  *   refilled from the block's ring of pending phonons and the batch's primaries; film
  *   entries and daughters appended to block buffers) and a film phase (every thread runs
  *   the waiting film cascades, their re-emissions appended to the ring), so an SM runs one
- *   code path at a time; ring_capacity: pending phonons per block (default 2^17).
+ *   code path at a time; ring_capacity: pending phonons per block (default 2^17) of a call
+ *   with a unit for every thread; a call with fewer units has a block on every SM all the
+ *   same, with rings of twice the same room per unit (4,096 at least).
  * form = 2: the warp pool, one persistent launch in which every warp runs its own film
  *   cascades between its transport steps; ring_capacity: pending phonons per warp (default
  *   1024).
@@ -545,8 +547,9 @@ int cmpmc_gpu_configure_phases(cmpmc_gpu_ctx* ctx, uint32_t phase_steps);
  *   the same substreams as form 1: the comparison point that shows what the FP32 form
  *   gains. Phonon-only batches with full film cascades (CMPMC_ERR_INVALID with charges or
  *   the Kaplan surrogate); ring entries 128 B, film records 80 B.
- * Rings are 80 B per entry; a ring (a power of two >= 64; 0 keeps the current value) that
- * overflows is grown 4x and the call rerun. All forms sample the same process; a daughter
+ * Rings are 80 B per entry. After an overflow of a ring (a power of two >= 64; 0 keeps the
+ * current value) the call reruns: with rings of full capacity where they had less, else with
+ * four times the capacity. All forms sample the same process; a daughter
  * runs on a substream drawn from its parent's in the pool forms, on the parent's own stream
  * in the host-driven form, so their hits agree in distribution, not bit for bit. */
 int cmpmc_gpu_configure_pool(cmpmc_gpu_ctx* ctx, int form, uint32_t ring_capacity);

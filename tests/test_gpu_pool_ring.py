@@ -18,3 +18,29 @@ def test_no_rerun_without_overflow(ge_lattice, form, n, ring):
     opt = cm.RunOptions(seed=31, form="batched_fp32", keep_hits=False, want_event_stats=True)
     for _ in range(3):
         assert eng.run_packed(packed, opt).kernel_launches == 5
+
+
+# Rings of 2,048 entries do not hold what 405 primaries of a block leave pending: the call reruns with
+# larger ones (more than the five launches), the next has them from the start, and a call of a few
+# units between them runs as it would have; a nearly full ring loses no phonon
+@pytest.mark.parametrize("form", [1, 3])
+def test_overflow_reruns_once_for_its_kind(ge_lattice, form):
+    import cmpmc_b200 as cm
+    from tests.test_gpu_spread import _same
+    det = cm.DetectorModel()
+    eng, ref = cm.SimulationEngine(ge_lattice, det), cm.SimulationEngine(ge_lattice, det)
+    eng.configure_pool(form, 2048)
+    ref.configure_pool(form, 1 << 17)
+    opt = cm.RunOptions(seed=3, form="batched_fp32", keep_hits=False, want_event_stats=True)
+    many = eng.generate(cm.workloads.mixed_energy, 600, 3)
+    few = eng.generate(cm.workloads.mixed_energy, 2, 4)
+    assert eng.run_packed(few, opt).kernel_launches == 5
+    first = eng.run_packed(many, opt)
+    assert first.kernel_launches > 5
+    want = ref.run_packed(many, opt)
+    assert want.kernel_launches == 5
+    _same(first, want)
+    assert eng.run_packed(few, opt).kernel_launches == 5
+    again = eng.run_packed(many, opt)
+    assert again.kernel_launches == 5
+    _same(again, want)
