@@ -360,11 +360,13 @@ CMPMC_HD double ekin_electron(const Lattice& L, int iv, V3 p) {
 CMPMC_HD double ekin_hole(const Lattice& L, V3 p) { return sqrt(norm2(p) + L.h_mass * L.h_mass) - L.h_mass; }
 // x / m with inv = 1 / m rounded: two residual corrections of x inv give the correctly rounded
 // quotient (P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", IBM J. Res. Dev. 34, 1990) for quotients in the normal range
+// processor", IBM J. Res. Dev. 34, 1990) for quotients in the normal range and for zeros. The
+// residual is taken as m q - x and its product subtracted, so that x = -0 stays -0: x - m q would
+// be +0 there.
 CMPMC_HD double div_by(double x, double m, double inv) {
     double q = x * inv;
-    q = crmath::fma_rn(crmath::fma_rn(-m, q, x), inv, q);
-    return crmath::fma_rn(crmath::fma_rn(-m, q, x), inv, q);
+    q = crmath::fma_rn(-crmath::fma_rn(m, q, -x), inv, q);
+    return crmath::fma_rn(-crmath::fma_rn(m, q, -x), inv, q);
 }
 // vel_electron with the reciprocals of the mass ratios at hand
 CMPMC_HD V3 vel_electron(const Lattice& L, V3 inv_mass, int iv, V3 p) {
