@@ -227,6 +227,7 @@ _SIG = {
     "cmpmc_cr_cos": (_f64, [_f64]),
     "cmpmc_copy_out": (_i32, [C.c_void_p, C.c_void_p, C.c_size_t]),
     "cmpmc_gpu_math_check": (_i32, [_i32, _u64, C.c_void_p, C.c_void_p]),
+    "cmpmc_gpu_math_eval": (_i32, [_i32, _i32, _u64, C.c_void_p, C.c_void_p, C.c_void_p]),
     "cmpmc_mesh_create": (_i32, [C.c_void_p, C.c_void_p, _u64, C.c_void_p, _u64, _f64, _f64,
                                  C.POINTER(C.c_void_p)]),
     "cmpmc_mesh_build_cartesian": (_i32, [_f64, _f64, _f64, _i32, _i32, _i32, C.c_void_p, C.c_void_p,

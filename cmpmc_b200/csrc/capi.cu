@@ -956,6 +956,21 @@ int cmpmc_gpu_math_check(int device, uint64_t n, const double* x, double* out) {
     return e == cudaSuccess ? CMPMC_OK : CMPMC_ERR_CUDA;
 }
 
+int cmpmc_gpu_math_eval(int device, int fn, uint64_t n, const double* x, const double* y, double* out) {
+    if (fn < CMPMC_MATH_LOG || fn > CMPMC_MATH_DIV || !x || !out || (fn == CMPMC_MATH_DIV && !y))
+        return CMPMC_ERR_INVALID;
+    if (cudaSetDevice(device) != cudaSuccess) return CMPMC_ERR_NO_DEVICE;
+    const uint64_t bytes = std::max<uint64_t>(n, 1) * 8;
+    double* dev = nullptr;  // x, y, out
+    cudaError_t e = cudaMalloc(&dev, 3 * bytes);
+    if (e == cudaSuccess) e = cudaMemcpy(dev, x, n * 8, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && fn == CMPMC_MATH_DIV) e = cudaMemcpy(dev + bytes / 8, y, n * 8, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && n) e = launch_math_eval(fn, n, dev, dev + bytes / 8, dev + bytes / 4);
+    if (e == cudaSuccess) e = cudaMemcpy(out, dev + bytes / 4, n * 8, cudaMemcpyDeviceToHost);
+    cudaFree(dev);
+    return e == cudaSuccess ? CMPMC_OK : CMPMC_ERR_CUDA;
+}
+
 int cmpmc_gpu_create(const cmpmc_lattice* lat, const cmpmc_detector* det, int device, cmpmc_gpu_ctx** out) {
     cmpmc_gpu_ctx* ctx = nullptr;
     if (!out) return fail(nullptr, CMPMC_ERR_INVALID, "out is NULL");

@@ -277,6 +277,7 @@ cudaError_t launch_batched_finish(const RunArgs& a, uint64_t n_events, const uin
                                   cmpmc_sim_stats* partials, cmpmc_sim_stats* ev_stats_out, cudaStream_t s,
                                   int* launches);
 cudaError_t launch_math_check(uint64_t n, const double* x, double* out);
+cudaError_t launch_math_eval(int fn, uint64_t n, const double* x, const double* y, double* out);
 // batched charge form: carriers (FP32 drift) filling the Luke-phonon queue, then the
 // phonon kernel over the queue entries; both add to per-event sinks
 cudaError_t launch_charges_fp32(const Lattice& L, const float* cdf_f, const Detector& D, const RunArgs& a,

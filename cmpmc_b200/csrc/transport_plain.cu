@@ -208,6 +208,25 @@ cudaError_t launch_math_check(uint64_t n, const double* x, double* out) {
     return cudaGetLastError();
 }
 
+__global__ void k_math_eval(int fn, uint64_t n, const double* __restrict__ x, const double* __restrict__ y,
+                            double* __restrict__ out) {
+    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
+         i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        switch (fn) {
+            case CMPMC_MATH_LOG: out[i] = crmath::log(x[i]); break;
+            case CMPMC_MATH_SIN: out[i] = crmath::sin(x[i]); break;
+            case CMPMC_MATH_COS: out[i] = crmath::cos(x[i]); break;
+            case CMPMC_MATH_EXP: out[i] = crmath::exp(x[i]); break;
+            default: out[i] = div_by(x[i], y[i], 1.0 / y[i]); break;
+        }
+    }
+}
+
+cudaError_t launch_math_eval(int fn, uint64_t n, const double* x, const double* y, double* out) {
+    k_math_eval<<<148, 256>>>(fn, n, x, y, out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_plain_fp64(const Lattice& L, const Detector& D, const RunArgs& a, int grid, int block,
                               cudaStream_t s) {
     if (a.ch_off) k_plain_fp64<true><<<grid, block, 0, s>>>(L, D, a);

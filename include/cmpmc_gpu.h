@@ -708,6 +708,16 @@ double cmpmc_cr_cos(double x);
 /* Evaluates the device's log, sin and cos on n host inputs and writes out[3*i+{0,1,2}]
  * (for checking that device and host agree bit for bit). */
 int cmpmc_gpu_math_check(int device, uint64_t n, const double* x, double* out);
+/* The same for one function at a time, each as the transport calls it by itself; CMPMC_MATH_DIV is
+ * x / y through the reciprocal of y (y: the divisors, unused otherwise). */
+enum {
+    CMPMC_MATH_LOG = 0,
+    CMPMC_MATH_SIN = 1,
+    CMPMC_MATH_COS = 2,
+    CMPMC_MATH_EXP = 3,
+    CMPMC_MATH_DIV = 4
+};
+int cmpmc_gpu_math_eval(int device, int fn, uint64_t n, const double* x, const double* y, double* out);
 
 /* Layout self-check for bindings: writes sizeof of the ABI structs in the order
  * phonon_track, charge_track, sensor_hit, sim_stats, crystal_config, film_config,
