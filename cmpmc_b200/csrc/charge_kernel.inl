@@ -2,16 +2,20 @@
 //   CHARGE_DEFER 0: a step's event (Luke emission, intervalley scatter, trap) is drawn at once;
 //   CHARGE_DEFER 1: it waits until a quarter of the warp's carriers wait for theirs, while the
 //                   others go on stepping.
-// One text for both, so that both do the same arithmetic in the same order (a template's two
-// instances were contracted into different multiply-adds, and a carrier that differs in one bit
-// takes another path).
+// A carrier that differs in one bit takes another path, and which form runs depends on the size of
+// the batch, so both have to round alike. One text for both makes that likely (a template's two
+// instances were contracted into different multiply-adds), not certain: tests/test_gpu_charge_forms.py
+// compares them over fields, masks, released energies and parked carriers. With open trapping
+// channels they differ in a trapped carrier's energy, and such crystals keep the first form
+// (charges_wait).
 //
 // A carrier is one serial chain of ~19,000 steps, so a step's instruction count is its latency
 // (few carriers) as well as its throughput (many). A step without an event (nine of ten) does
 // only what the next one reads: |k| once, the velocity of the rates only where a trapping
 // channel is open, no kinetic energy (the intervalley threshold is decided by |k|), and no
-// exit point for a carrier far from every wall. 4,000 carriers 101 -> 66 ms, 100,000 carriers
-// 182 -> 134 ms, the carriers and phonons of 64 light recoils 117 -> 88 ms.
+// exit point for a carrier far from every wall. 4,000 carriers (the first form) 101 -> 66 ms, the
+// carriers and phonons of 64 light recoils 117 -> 88 ms; 100,000 carriers 182 -> 134 ms in the first
+// form, 99 ms in the waiting one that runs at that size.
 // (128, 5): 96 registers, five blocks per SM (with the step as it was, pair drift of 200,000
 // events 467 -> 431 ms against (128, 4) at 104 registers; (128, 6) at 80 registers 432 ms)
 __global__ void __launch_bounds__(128, 5) CHARGE_KERNEL(const __grid_constant__ FCLat Lp,
@@ -237,22 +241,22 @@ __global__ void __launch_bounds__(128, 5) CHARGE_KERNEL(const __grid_constant__ 
                     ++st.crefl;
                     c.pos = c.pos + bh.n * kNudge;
                     // ChargePhysics::reflect_at_boundary (charge_transport.hpp:203-241)
-                    bool done = false;
+                    bool mirrored = false;
                     if (k.g.u() < s.prob_spec) {
                         const F3 kd = funit(c.p);
                         const F3 kr = funit(kd - bh.n * (2.0f * fdot(kd, bh.n)));
                         if (c.type == 2) {
                             c.p = kr * fnorm(c.p);
-                            done = true;
+                            mirrored = true;
                         } else {
                             const F3 pt = ekin_to_p_e(L, c.valley, kr, c.ekin);
                             if (fdot(vel_of(L, 1, c.valley, pt), bh.n) > 1e-6f) {
                                 c.p = pt;
-                                done = true;
+                                mirrored = true;
                             }
                         }
                     }
-                    if (!done) {
+                    if (!mirrored) {
                         const F3 e1 = forth(bh.n);
                         const F3 e2 = fcross(bh.n, e1);
                         if (c.type == 2) {
