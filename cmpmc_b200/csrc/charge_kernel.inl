@@ -206,12 +206,7 @@ __global__ void __launch_bounds__(128, 5) CHARGE_KERNEL(const __grid_constant__ 
         const F3 v_mid = vel_of(L, c.type, c.valley, p_mid);
         const float v_mag = fnorm(v_mid);
         const float d_step = v_mag * dt;
-        // a carrier whose distance to every wall is over twice the step (plus an edge far above
-        // the rounding of the exit point) cannot reach one; anything not finite takes the test
-        const float reach = 2.0f * d_step + D.edge;
-        const float r_in = D.R - reach;
-        const bool inside = r_in > 0.0f && fabsf(c.pos.z) < D.H - reach &&
-                            c.pos.x * c.pos.x + c.pos.y * c.pos.y < r_in * r_in;
+        const bool inside = clear_of_walls(D.R, D.H, D.edge, c.pos.x, c.pos.y, c.pos.z, d_step);
         if (!inside && v_mag > 1e-6f) {
             const F3 v_dir = v_mid * (1.0f / v_mag);
             const FBHit bh = fexit(D.R, D.H, c.pos, v_dir);

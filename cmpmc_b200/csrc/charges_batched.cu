@@ -23,6 +23,7 @@
 #define CMPMC_DEVICE_FAST_MATH 1
 #include <algorithm>
 
+#include "charge_shortcuts.cuh"
 #include "device.cuh"
 #include "fp32.cuh"
 
@@ -548,10 +549,9 @@ FCLat make_fclat(const Lattice& L, const float* cdf_f, const Detector& D) {
     f.n_valleys = L.n_valleys;
     f.iv_model = L.iv_model;
     f.iv_min = static_cast<float>(L.iv_min_energy);
-    // |k| of an electron at iv_min (1 -+ 1e-3): far outside the rounding of either comparison
-    auto k_at = [&](double e) { return static_cast<float>(sqrt(e * e + 2.0 * e * L.e_cond_mass) / kHbarC); };
-    f.k_iv_lo = L.iv_min_energy > 0.0 ? k_at(L.iv_min_energy * 0.999) : -1.0f;
-    f.k_iv_hi = L.iv_min_energy > 0.0 ? k_at(L.iv_min_energy * 1.001) : kInfF;
+    const KBand band = k_band(L.iv_min_energy, L.e_cond_mass);
+    f.k_iv_lo = band.lo;
+    f.k_iv_hi = band.hi;
     f.iv_qrate = static_cast<float>(L.iv_quad_rate);
     f.iv_qfield = static_cast<float>(L.iv_quad_field);
     f.iv_qpow_half = static_cast<float>(0.5 * L.iv_quad_power);
@@ -590,7 +590,7 @@ FCDet make_fcdet(const Detector& D, const MeshView32& mesh, const Lattice& L) {
         f.surf[i].pads = D.surf[i].pads;
         f.surf[i].release = (D.charge_release == 1 || (D.charge_release == 2 && D.surf[i].has_film)) ? 1 : 0;
     }
-    f.edge = 1e-4f * (f.R + f.H);
+    f.edge = wall_edge(f.R, f.H);
     f.dt_cap = static_cast<float>(D.charge_dt_cap_s);
     const bool second = (D.charge_stepping == 1);
     f.dk_frac = static_cast<float>(second ? D.charge_sampling_dk_frac : D.charge_max_dk_frac);
