@@ -130,8 +130,10 @@ struct PlainCtx {
 // power at every step), sine and cosine come from one reduction, log and exp have no division,
 // the transcendentals and the rare branches are out of line, and a phonon-only run takes a
 // kernel without the carriers' loop (kCharges). 2,000 phonon events 84 -> 58 ms, 203 mixed
-// events 234 -> 122 ms. Blocks per SM (phonons / mixed, ms): two 68 / 122, three 58 / 137, four
-// 63 / 144, five 67 / 152: more warps pay for phonons, registers without spills for carriers.
+// events 234 -> 122 ms. Blocks per SM, 2,000 phonon events: two 68 ms, three 58, four 63, five 67.
+// With carriers registers without spills are worth more than a third block, also where the events
+// fill the chip (mixed events, two / three blocks): 203 128 / 146 ms, 1,400 218 / 253, 2,800 328 /
+// 325, 4,000 360 / 447, 10,000 586 / 635.
 template <bool kCharges>
 __global__ void __launch_bounds__(128, kCharges ? 2 : 3) k_plain_fp64(const __grid_constant__ Lattice L,
                                                     const __grid_constant__ Detector D,
